@@ -100,7 +100,7 @@ __device__ __forceinline__ float rl_udotu(float ux, float uy, float uz) {
 // I = 0..N-1 without relying on the optimiser to unroll.
 template <int I> struct IC { static constexpr int value = I; };
 template <int B, int E, class F>
-__device__ __forceinline__ void static_for(F&& f) {
+__host__ __device__ __forceinline__ void static_for(F&& f) {
   if constexpr (B < E) {
     f(IC<B>{});
     static_for<B + 1, E>(f);

@@ -153,7 +153,7 @@ bool setup_physics(Ctx& c, const lbm_desc& d) {
   g.nx = d.nx; g.ny = d.ny; g.nz = d.nz;
   g.n = (size_t)d.nx * d.ny * d.nz;
   for (int a = 0; a < 3; ++a) g.per[a] = d.periodic[a];
-  g.px = g.per[0] ? g.nx : (int)round_up((size_t)g.nx + 1, 8);
+  g.px = (int)round_up((size_t)g.nx + (g.per[0] ? 0 : 1), 8);
   g.gy = g.per[1] ? 0 : 1;
   g.gz = g.per[2] ? 0 : 1;
   g.py = g.ny + 2 * g.gy;
@@ -546,6 +546,7 @@ int lbm_sync(lbm_ctx* c) {
   CK(cudaStreamSynchronize(c->stream), "sync");
   if (st) {
     CK(cudaMemsetAsync(c->status, 0, sizeof(unsigned), c->stream), "reset status");
+    if (st & 4u) return fail(c, LBM_ERR_TIMEOUT, "a step kernel's wait for its row copies gave up");
     if (st & 2u)
       return fail(c, LBM_ERR_TIMEOUT, "the closure's tensor-core MMA wait gave up (nodes fell back to Smagorinsky)");
     return fail(c, LBM_ERR_NONFINITE, "non-finite value or rho <= 0 at a fluid node");

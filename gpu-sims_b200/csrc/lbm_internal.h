@@ -112,6 +112,10 @@ cudaError_t phys_step(const Ctx& c, int parity, bool write_moments, cudaStream_t
 cudaError_t phys_step_f32(const Ctx& c, int parity, bool write_moments, cudaStream_t s);
 cudaError_t phys_step_f16(const Ctx& c, int parity, bool write_moments, cudaStream_t s);
 cudaError_t phys_step_bf16(const Ctx& c, int parity, bool write_moments, cudaStream_t s);
+// the row-tile form of a step without the learned closure (phys_rows.cuh)
+cudaError_t phys_rows_f32(const Ctx& c, int parity, bool write_moments, cudaStream_t s);
+cudaError_t phys_rows_f16(const Ctx& c, int parity, bool write_moments, cudaStream_t s);
+cudaError_t phys_rows_bf16(const Ctx& c, int parity, bool write_moments, cudaStream_t s);
 cudaError_t phys_step_clo_f32(const Ctx& c, int parity, bool write_moments, cudaStream_t s);
 cudaError_t phys_step_clo_f16(const Ctx& c, int parity, bool write_moments, cudaStream_t s);
 cudaError_t phys_step_clo_bf16(const Ctx& c, int parity, bool write_moments, cudaStream_t s);

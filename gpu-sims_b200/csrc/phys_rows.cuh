@@ -1,0 +1,705 @@
+// Row-tile step of the physics mode: persistent blocks that stream whole rows
+// through shared memory with bulk copies, so that the collision threads do no
+// address arithmetic at all.
+//
+// A tile is R consecutive rows of one z-plane.  In each of the 19 slot arrays
+// its values are one contiguous run of R * px elements, fetched by one
+// cp.async.bulk and written back by one (two where a row at a y face comes
+// from another place).  One producer warp issues them and resolves everything that depends on the row only: the parity, the periodic
+// wraps, and the half-way bounce-back of the y and z faces (the same location
+// of the pair's other slot array).  The x faces' bounce-back values (one
+// element per row and array) arrive by 4-byte cp.async next to the rows.
+// Consumer threads own two x-adjacent nodes for the whole launch; every access
+// is a fixed offset from a few per-thread bases, the slots at x+1 of the
+// c_x = +1 pairs included.
+//
+// What bounds it.  The row kernels (phys_step_launch.cuh) spend 462 thread
+// instructions a node on fp16 storage, half of them addresses, face predicates
+// and shuffles, and are bound by their issue; here it is 330, the collision most
+// of them, and HBM is the bound of wide grids.  B200, GLUPS (row kernels in
+// brackets): fp16 channel 512x128x128 69 = 5.3 TB/s (54), periodic TRT 256^3 76 =
+// 5.9 TB/s (57), open duct 512x128x128 67 (51), cavity 160^3 62 (44), 161x97x75
+// with Smagorinsky 34.6 (26.2); fp32 channel 41.2 = 6.3 TB/s (39.4), duct 39.1
+// (34.9), cavity 160^3 37.1 (33.6), 101^3 38.9 (29.3), 161x97x75 with Smagorinsky
+// 30.8 (25.1).
+// Four service warps rather than one: each copy is a serial handful of
+// instructions, and one warp issuing all 38 of a tile held the block back
+// (channel fp16 38.7).  A tile of about 512 nodes keeps the copies long (1 KB
+// and up), and five stages of it fit two blocks per SM (2-byte storage).
+//
+// In place.  Every slot element belongs to one node per launch (phys_kernels.cu),
+// so a row of S[1-P] belongs to its own tile and a row of S[P] to the tile of
+// the row it is the forward neighbour of; tiles never write each other's rows.
+// Elements nobody owns (solid nodes' slots, row padding, x = 0 of the c_x = +1
+// pairs beside a wall) are written back as they were read.  Where a face row
+// was read from the pair's other array, the elements left unwritten are slots
+// whose reader would lie outside the box.
+#pragma once
+#include "phys_step.cuh"
+
+namespace lbm {
+namespace {
+
+constexpr int ROWS_CAP = 576;    // elements of a tile in one slot array
+constexpr int ROWS_MAXR = 16;    // rows of a tile
+constexpr int ROWS_CONS = 256;   // consumer threads
+constexpr int ROWS_SERV = 4;     // service warps, which issue the copies
+constexpr int ROWS_MAXST = 5;
+// polls of a wait (each try_wait suspends for a while) before the block gives up
+constexpr uint32_t ROWS_WAIT_LIMIT = 1u << 22;
+
+// One array's part of a stage: the tile's elements, then a 4-byte slot per
+// row for the x face's value.
+template <int PREC>
+constexpr int rows_region() {
+  return ROWS_CAP * (int)sizeof(typename Store<PREC>::T) + ROWS_MAXR * 4;
+}
+template <int PREC>
+constexpr int rows_stage() {
+  return Q * rows_region<PREC>();
+}
+static_assert(rows_region<LBM_PREC_F32>() % 16 == 0 && rows_region<LBM_PREC_F16S>() % 16 == 0,
+              "bulk copies start on 16-byte boundaries");
+
+constexpr int ROWS_THREADS = 32 * ROWS_SERV + ROWS_CONS;
+// Blocks per SM.  One for Smagorinsky, whose collision spills at 96 registers
+// (periodic 256^3 fp32 41.1 GLUPS against 27.1 with two, 128^3 fp16 49.9 against
+// 42.8).
+template <int PREC, int SGS>
+constexpr int rows_blocks() {
+  return SGS ? 1 : 2;
+}
+// Two blocks of 12 warps leave 80 registers a thread at launch (384 * 80 =
+// 30,720 a block); the service warpgroup hands its share on:
+// 128 * 40 + 256 * 96 = 29,696.
+constexpr int ROWS_REGS_SERV = 40, ROWS_REGS_CONS = 96;
+static_assert(128 * ROWS_REGS_SERV + ROWS_CONS * ROWS_REGS_CONS <= ROWS_THREADS * 80, "registers of a block");
+
+struct RowTiles {
+  int R;            // rows per tile
+  int tpr;          // consumer threads per row, two nodes each
+  int tiles_y;      // tiles per z-plane
+  uint32_t ntiles;
+  int stages;
+};
+
+__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive_tx(uint32_t bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
+  uint32_t done;
+  asm volatile(
+      "{\n\t.reg .pred P1;\n\tmbarrier.try_wait.parity.shared::cta.b64 P1, [%1], %2;\n\t"
+      "selp.b32 %0, 1, 0, P1;\n\t}\n"
+      : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+  return done != 0;
+}
+// Bounded wait: false when it ran out or another warp of the block gave up.
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile uint32_t* abort) {
+  if (mbar_try(bar, parity)) return true;
+  for (uint32_t i = 0; i < ROWS_WAIT_LIMIT; ++i) {
+    if (mbar_try(bar, parity)) return true;
+    if (*abort) return false;
+  }
+  return false;
+}
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+               ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void bulk_store(void* dst, uint32_t src, uint32_t bytes) {
+  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;"
+               ::"l"(dst), "r"(src), "r"(bytes) : "memory");
+}
+
+// A tile of a walk over the grid: first, first + stride, ... in row order.
+struct RowWalk {
+  int ty, z;      // tile within its plane, plane
+  int dty, dz;    // the stride in both
+  __host__ __device__ __forceinline__ void start(uint32_t first, uint32_t stride, int tiles_y) {
+    z = (int)(first / (uint32_t)tiles_y);
+    ty = (int)(first - (uint32_t)z * (uint32_t)tiles_y);
+    dz = (int)(stride / (uint32_t)tiles_y);
+    dty = (int)(stride - (uint32_t)dz * (uint32_t)tiles_y);
+  }
+  __host__ __device__ __forceinline__ void next(int tiles_y) {
+    ty += dty;
+    z += dz;
+    if (ty >= tiles_y) {
+      ty -= tiles_y;
+      ++z;
+    }
+  }
+};
+
+// Row shift of array k's tile rows: (cy, cz) of the pair for Y arrays (even k),
+// 0 for X arrays and the rest array.
+__host__ __device__ __forceinline__ void array_dir(int k, int& cya, int& czz) {
+  // c_y + 1 and c_z + 1 of the nine pairs' forward vectors, two bits each
+  constexpr uint32_t CY = [] {
+    uint32_t v = 0;
+    for (int q = 0; q < 9; ++q) v |= (uint32_t)(cy(pair_a(q)) + 1) << (2 * q);
+    return v;
+  }();
+  constexpr uint32_t CZ = [] {
+    uint32_t v = 0;
+    for (int q = 0; q < 9; ++q) v |= (uint32_t)(cz(pair_a(q)) + 1) << (2 * q);
+    return v;
+  }();
+  const int q = k > 0 ? (k - 1) >> 1 : 0;
+  cya = k > 0 ? (int)((CY >> (2 * q)) & 3u) - 1 : 0;
+  czz = k > 0 ? (int)((CZ >> (2 * q)) & 3u) - 1 : 0;
+}
+
+// Element offset (from the tile's first element in array 0) of array k's rows
+// in a tile away from the y and z faces: where they are loaded from and stored
+// to.  X arrays: S[1-P](n); Y arrays: S[P](n + d).
+__host__ __device__ __forceinline__ ptrdiff_t array_offset(const PhysGeom& G, int k, int P) {
+  if (k == 0) return 0;
+  int dy, dz;
+  array_dir(k, dy, dz);
+  const int s0 = 1 + ((k - 1) & ~1);
+  const bool Y = !(k & 1);
+  const ptrdiff_t arr = (ptrdiff_t)((Y ? P : 1 - P) + s0) * (ptrdiff_t)G.slot_stride;
+  return Y ? arr + (ptrdiff_t)dy * G.px + (ptrdiff_t)dz * (ptrdiff_t)G.pxy : arr;
+}
+
+// Array k's rows of any tile: calls copy(element offset from the tile's first
+// element in array 0, first row, rows) for every run.  LOAD: where the streamed
+// values come from (the pair's other array at a bounce-back face); else where
+// the results go.
+template <bool LOAD, class F>
+__host__ __device__ __forceinline__ void face_runs(const PhysGeom& G, int P, int k, int y0, int z, int rows, F&& copy) {
+  const ptrdiff_t SS = (ptrdiff_t)G.slot_stride;
+  ptrdiff_t m = array_offset(G, k, P);
+  int dy, dz;
+  array_dir(k, dy, dz);
+  const bool Y = k > 0 && !(k & 1);
+  // to the pair's other array: S[P] <-> S[1-P]
+  const ptrdiff_t other = k == 0 ? 0 : ((Y ? P : 1 - P) ? -SS : SS);
+  // the faces that n + d (Y) or n - d (X) may cross
+  const int ey = Y ? dy : -dy, ez = Y ? dz : -dz;
+  const bool fy = (ey > 0 && y0 + rows == G.ny) || (ey < 0 && y0 == 0);
+  const bool fz = (ez > 0 && z == G.nz - 1) || (ez < 0 && z == 0);
+  const ptrdiff_t plain = m;
+  if (fz) {
+    if (!G.per[2]) m += LOAD ? other : 0;
+    else if (Y) m -= (ptrdiff_t)ez * (ptrdiff_t)G.pxy * G.nz;
+  }
+  const int r = ey > 0 ? rows - 1 : 0;  // the row at the y face
+  ptrdiff_t e = m;
+  bool own = false;                     // that row comes from (goes) elsewhere
+  if (fy) {
+    if (!G.per[1]) {
+      own = LOAD;
+      e = plain + other;
+      // a corner link that also wraps in z keeps its wrap
+      if (fz && G.per[2] && Y) e -= (ptrdiff_t)ez * (ptrdiff_t)G.pxy * G.nz;
+    } else if (Y) {
+      own = true;
+      e = m - (ptrdiff_t)ey * (ptrdiff_t)G.px * G.ny;
+    }
+  }
+  if (!own) {
+    copy(m, 0, rows);
+    return;
+  }
+  copy(e + (ptrdiff_t)r * G.px, r, 1);
+  if (rows > 1) {
+    const int f = r == 0 ? 1 : 0;
+    copy(m + (ptrdiff_t)f * G.px, f, rows - 1);
+  }
+}
+
+// Entry i of a tile's x-face values (10 per row): its source element's word and
+// its place in the stage.  f_a of x = 0 is S[P](0), f_b of x = nx-1 is
+// S[1-P](nx) of the forward row.
+template <int PREC>
+__host__ __device__ __forceinline__ const typename Store<PREC>::T* row_side(const PhysGeom& G, const void* pop, int P,
+                                                                            int i, int y0, int z, uint32_t& off) {
+  using T = typename Store<PREC>::T;
+  const int r = i / 10, e = i - 10 * r, k = e >> 1;
+  const int pi = k == 0 ? 0 : k + 2;  // the pairs with c_x = +1: 0, 3, 4, 5, 6
+  const int a = pair_a(pi);
+  const T* s0 = reinterpret_cast<const T*>(pop) + (size_t)(1 + 2 * pi) * G.slot_stride;
+  const T* s1 = s0 + G.slot_stride;
+  off = (uint32_t)(1 + 2 * pi + (e & 1)) * rows_region<PREC>() + ROWS_CAP * (uint32_t)sizeof(T) + 4u * (uint32_t)r;
+  if (!(e & 1)) return (P ? s1 : s0) + lin(G, 0, y0 + r, z);
+  int yn = y0 + r + cy(a), zn = z + cz(a);
+  if (G.per[1]) yn = yn < 0 ? yn + G.ny : (yn >= G.ny ? yn - G.ny : yn);
+  if (G.per[2]) zn = zn < 0 ? zn + G.nz : (zn >= G.nz ? zn - G.nz : zn);
+  return (P ? s0 : s1) + lin(G, sizeof(T) == 2 ? G.nx & ~1 : G.nx, yn, zn);
+}
+
+// The same entry of row 0 of a tile away from the y and z faces, from the tile's
+// first element in array 0.
+template <int PREC>
+__host__ __device__ __forceinline__ ptrdiff_t side_offset(const PhysGeom& G, int P, int e, uint32_t& off) {
+  const int k = e >> 1, pi = k == 0 ? 0 : k + 2;
+  constexpr int EB = sizeof(typename Store<PREC>::T);
+  off = (uint32_t)(1 + 2 * pi + (e & 1)) * rows_region<PREC>() + ROWS_CAP * (uint32_t)EB;
+  if (!(e & 1)) return (ptrdiff_t)(1 + 2 * pi + P) * (ptrdiff_t)G.slot_stride;
+  int dy, dz;
+  array_dir(2 + 2 * pi, dy, dz);
+  return (ptrdiff_t)(2 + 2 * pi - P) * (ptrdiff_t)G.slot_stride + (ptrdiff_t)dy * G.px +
+         (ptrdiff_t)dz * (ptrdiff_t)G.pxy + (EB == 2 ? G.nx & ~1 : G.nx);
+}
+
+// A service warp.  One lane issues the copies of its arrays: their operands are
+// then uniform over the warp, and each costs a handful of instructions.
+template <int PREC>
+__device__ __forceinline__ void rows_service(const PhysGeom& G, const RowTiles& rt, void* pop, int P, int part,
+                                              uint32_t stage0, uint32_t full0, uint32_t done0,
+                                              volatile uint32_t* abort, unsigned* status) {
+  using T = typename Store<PREC>::T;
+  constexpr uint32_t EB = sizeof(T);
+  constexpr int NA = (Q + ROWS_SERV - 1) / ROWS_SERV;  // arrays of a service warp: part, part + ROWS_SERV, ...
+  const int lane = threadIdx.x & 31;
+  char* base = reinterpret_cast<char*>(pop);
+  const uint32_t row_bytes = (uint32_t)G.px * EB;
+  const uint32_t n = rt.ntiles <= blockIdx.x ? 0u : (rt.ntiles - blockIdx.x + gridDim.x - 1) / gridDim.x;
+  const uint32_t stages = (uint32_t)rt.stages;
+  const uint32_t arrays = (uint32_t)((Q + ROWS_SERV - 1 - part) / ROWS_SERV);
+  ptrdiff_t off[NA];
+#pragma unroll
+  for (int i = 0; i < NA; ++i) off[i] = array_offset(G, min(part + ROWS_SERV * i, Q - 1), P) * (ptrdiff_t)EB;
+  const uint32_t region0 = (uint32_t)part * rows_region<PREC>();
+  // this lane's x-face value of a row: where it lies from the row's first
+  // element in array 0 (tiles away from the y and z faces), and its place
+  const int side_row = lane < 30 ? lane / 10 : ROWS_MAXR, side_e = lane % 10;
+  uint32_t side_dst;
+  const ptrdiff_t side_src = side_offset<PREC>(G, P, side_e, side_dst) * (ptrdiff_t)EB;
+  auto inner = [&](int y0, int z, int rows) { return y0 > 0 && y0 + rows < G.ny && z > 0 && z < G.nz - 1; };
+  RowWalk wl, ws;  // of the loads and of the stores
+  wl.start(blockIdx.x, gridDim.x, rt.tiles_y);
+  ws = wl;
+  auto load = [&](uint32_t s) {
+    const int z = wl.z, y0 = wl.ty * rt.R, rows = min(rt.R, G.ny - y0);
+    const uint32_t st = stage0 + s * rows_stage<PREC>(), bar = full0 + 8 * s;
+    if (lane == 0) {
+      char* at = base + lin(G, 0, y0, z) * EB;
+      const uint32_t bytes = (uint32_t)rows * row_bytes;
+      mbar_arrive_tx(bar, bytes * arrays);
+      if (inner(y0, z, rows)) {
+#pragma unroll
+        for (int i = 0; i < NA; ++i)
+          if (part + ROWS_SERV * i < Q)
+            bulk_load(st + region0 + ROWS_SERV * i * rows_region<PREC>(), at + off[i], bytes, bar);
+      } else {
+#pragma unroll 1
+        for (int k = part; k < Q; k += ROWS_SERV)
+          face_runs<true>(G, P, k, y0, z, rows, [&](ptrdiff_t el, int r, int cnt) {
+            bulk_load(st + k * rows_region<PREC>() + (uint32_t)r * row_bytes, at + el * (ptrdiff_t)EB,
+                      (uint32_t)cnt * row_bytes, bar);
+          });
+      }
+    }
+    __syncwarp();
+    if (!G.per[0]) {
+      // ten lanes a row, three rows a warp
+      const char* at = base + lin(G, 0, y0, z) * EB + side_src;
+      const bool in = inner(y0, z, rows);
+      for (int r = 3 * part + side_row; r < rows; r += 3 * ROWS_SERV) {
+        const char* src = at + (uint32_t)r * row_bytes;
+        uint32_t o = side_dst + 4u * (uint32_t)r;
+        if (!in) src = reinterpret_cast<const char*>(row_side<PREC>(G, pop, P, 10 * r + side_e, y0, z, o));
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(st + o), "l"(src) : "memory");
+      }
+      asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
+    }
+    wl.next(rt.tiles_y);
+  };
+  const uint32_t ahead = min(stages, n);
+  #pragma unroll 1
+  for (uint32_t j = 0; j < ahead; ++j) load(j);
+  uint32_t loaded = ahead, s = 0, ph = 0, prev = 0;
+  for (uint32_t j = 0; j < n; ++j) {
+    const bool ok = mbar_wait(done0 + 8 * s, ph, abort);
+    if (!__all_sync(FULL, ok)) {
+      if (lane == 0) {
+        *abort = 1u;
+        atomicOr(status, 4u);
+      }
+      break;
+    }
+    const int z = ws.z, y0 = ws.ty * rt.R, rows = min(rt.R, G.ny - y0);
+    if (lane == 0) {
+      const uint32_t st = stage0 + s * rows_stage<PREC>();
+      char* at = base + lin(G, 0, y0, z) * EB;
+      if (inner(y0, z, rows)) {
+#pragma unroll
+        for (int i = 0; i < NA; ++i)
+          if (part + ROWS_SERV * i < Q)
+            bulk_store(at + off[i], st + region0 + ROWS_SERV * i * rows_region<PREC>(), (uint32_t)rows * row_bytes);
+      } else {
+#pragma unroll 1
+        for (int k = part; k < Q; k += ROWS_SERV)
+          face_runs<false>(G, P, k, y0, z, rows, [&](ptrdiff_t el, int r, int cnt) {
+            bulk_store(at + el * (ptrdiff_t)EB, st + k * rows_region<PREC>() + (uint32_t)r * row_bytes,
+                       (uint32_t)cnt * row_bytes);
+          });
+      }
+      asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+      // refill the stage whose stores have left it: the previous tile's, or with
+      // two stages this tile's own
+      if (stages > 2) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+      else asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+    }
+    __syncwarp();
+    ws.next(rt.tiles_y);
+    if (stages <= 2) prev = s;
+    if ((j > 0 || stages <= 2) && loaded < n) {
+      load(prev);
+      ++loaded;
+    }
+    prev = s;
+    if (++s == stages) {
+      s = 0;
+      ph ^= 1u;
+    }
+  }
+  if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+  if (*abort) {
+    // leave no copy in flight: the loads that no consumer waited for
+    for (uint32_t j = loaded > stages ? loaded - stages : 0u; j < loaded; ++j)
+      for (uint32_t i = 0; i < ROWS_WAIT_LIMIT; ++i)
+        if (mbar_try(full0 + 8 * (j % stages), (j / stages) & 1u)) break;
+  }
+}
+
+// One pair of nodes' step on a landed tile: stream from, and collide into, the
+// stage at st.
+struct RowPair {
+  int row, x;              // row within the tile, x of node A
+  bool active;             // the thread has a pair
+  uint32_t xo;             // byte offset of node A's element (X slots and c_x = 0 Y slots)
+  uint32_t lo;             // f_a of node A for the c_x = +1 pairs (x face: the side slot)
+  uint32_t yA, yB;         // their f_b of nodes A and B
+  uint32_t wA, wB;         // ... and where f*_a of A and B goes
+};
+
+template <int PREC>
+__host__ __device__ __forceinline__ RowPair row_pair(const PhysGeom& G, int R, int tpr, int tid) {
+  constexpr uint32_t EB = sizeof(typename Store<PREC>::T);
+  RowPair q;
+  q.row = tid / tpr;
+  q.active = q.row < R;
+  if (!q.active) q.row = 0;
+  q.x = q.active ? 2 * (tid - q.row * tpr) : 0;
+  const uint32_t r0 = (uint32_t)q.row * (uint32_t)G.px * EB;
+  const uint32_t side = ROWS_CAP * EB + 4 * (uint32_t)q.row;
+  q.xo = r0 + (uint32_t)q.x * EB;
+  q.lo = (!G.per[0] && q.x == 0) ? side : q.xo;
+  q.yA = q.wA = q.xo + EB;
+  q.yB = q.wB = q.xo + 2 * EB;
+  if (q.x == G.nx - 1) {
+    if (G.per[0]) q.yA = q.wA = r0;
+    else q.yA = side + (EB == 2 && (G.nx & 1) ? 2u : 0u);
+    q.yB = q.wB = q.xo + EB;  // node B does not exist
+  } else if (q.x + 1 == G.nx - 1) {
+    if (G.per[0]) q.yB = q.wB = r0;
+    else q.yB = side;  // nx even: the low half of its word
+  }
+  return q;
+}
+
+template <int PREC, int COLL, int SGS, bool FORCE, bool WRITE_MOMENTS, bool OPEN>
+__device__ __forceinline__ void row_pair_step(const PhysParams& p, uint8_t* __restrict__ st, const RowPair& q,
+                                              void* __restrict__ pop_v, const uint32_t* __restrict__ links,
+                                              float* __restrict__ rho_o, float* __restrict__ u_o,
+                                              unsigned* __restrict__ status, int y, int z, uint32_t fl2, int P) {
+  using S = Store<PREC>;
+  using V2 = Vec2<PREC>;
+  using T = typename S::T;
+  constexpr int REG = rows_region<PREC>();
+  const PhysGeom& G = p.g;
+  const int x = q.x;
+  auto el = [&](int region, uint32_t off) -> T* { return reinterpret_cast<T*>(st + region * REG + off); };
+  auto one = [&](int region, uint32_t off) { return S::raw_ld(el(region, off), 0); };
+  auto two = [&](int region) {
+    const typename V2::V r = V2::ld(el(region, q.xo), 0);
+    return make_float2(V2::lo(r), V2::hi(r));
+  };
+  float2 g[Q];  // .x = node A, .y = node B
+  g[0] = two(0);
+  static_for<0, 9>([&](auto PI) {
+    constexpr int pi = decltype(PI)::value;
+    constexpr int a = pair_a(pi), b = pair_b(pi);
+    if constexpr (cx(a) == 0) {
+      g[a] = two(1 + 2 * pi);
+      g[b] = two(2 + 2 * pi);
+    } else {
+      g[a] = make_float2(one(1 + 2 * pi, q.lo), one(1 + 2 * pi, q.xo + (uint32_t)sizeof(T)));
+      g[b] = make_float2(one(2 + 2 * pi, q.yA), one(2 + 2 * pi, q.yB));
+    }
+  });
+  const uint32_t nid = (uint32_t)x + (uint32_t)G.nx * ((uint32_t)y + (uint32_t)G.ny * (uint32_t)z);
+  const uint32_t flA = fl2 & 0xffu, flB = fl2 >> 8;
+  const bool fluidA = !(flA & FLAG_SOLID), fluidB = !(flB & FLAG_SOLID);
+  if (p.any_moving_wall && near_moving(p, x, x + 1 < G.nx ? x + 1 : x, y, z)) {
+    auto faces = [&](int xx, auto sel) {
+      constexpr bool B = decltype(sel)::value != 0;
+      const bool xlo = !G.per[0] && xx == 0, xhi = !G.per[0] && xx == G.nx - 1;
+      const bool ylo = !G.per[1] && y == 0, yhi = !G.per[1] && y == G.ny - 1;
+      const bool zlo = !G.per[2] && z == 0, zhi = !G.per[2] && z == G.nz - 1;
+      static_for<0, 9>([&](auto PI) {
+        constexpr int pi = decltype(PI)::value;
+        constexpr int a = pair_a(pi), b = pair_b(pi);
+        constexpr int DX = cx(a), DY = cy(a), DZ = cz(a);
+        const bool fwd = (DX > 0 && xhi) || (DY > 0 && yhi) || (DY < 0 && ylo) || (DZ > 0 && zhi) || (DZ < 0 && zlo);
+        const bool bwd = (DX > 0 && xlo) || (DY > 0 && ylo) || (DY < 0 && yhi) || (DZ > 0 && zlo) || (DZ < 0 && zhi);
+        float& va = B ? g[a].y : g[a].x;
+        float& vb = B ? g[b].y : g[b].x;
+        if (bwd) va = fmaf(S::SC, wall_term<a>(p, xx, y, z), va);
+        if (fwd) vb = fmaf(S::SC, wall_term<b>(p, xx, y, z), vb);
+      });
+    };
+    faces(x, IC<0>{});
+    if (x + 1 < G.nx) faces(x + 1, IC<1>{});
+  }
+  // links into interior solids: their bounce-back slots are nobody's this
+  // launch, so they are read from global memory
+  auto solid_fix = [&](int xx, auto sel) {
+    constexpr bool B = decltype(sel)::value != 0;
+    const T* pop = reinterpret_cast<const T*>(pop_v);
+    const uint32_t Lk = links[nid + (B ? 1 : 0)];
+    const uint32_t ln = lin32(G, xx, y, z);
+    const Wrap w = wrap_terms(G, xx, y, z);
+    const bool xlo = !G.per[0] && xx == 0, xhi = !G.per[0] && xx == G.nx - 1;
+    const bool ylo = !G.per[1] && y == 0, yhi = !G.per[1] && y == G.ny - 1;
+    const bool zlo = !G.per[2] && z == 0, zhi = !G.per[2] && z == G.nz - 1;
+    static_for<0, 9>([&](auto PI) {
+      constexpr int pi = decltype(PI)::value;
+      constexpr int a = pair_a(pi), b = pair_b(pi);
+      constexpr int DX = cx(a), DY = cy(a), DZ = cz(a);
+      const T* s0 = pop + (size_t)(1 + 2 * pi) * G.slot_stride;
+      const T *sP = P ? s0 + G.slot_stride : s0, *sQ = P ? s0 : s0 + G.slot_stride;
+      const bool fwd = (DX > 0 && xhi) || (DY > 0 && yhi) || (DY < 0 && ylo) || (DZ > 0 && zhi) || (DZ < 0 && zlo);
+      const bool bwd = (DX > 0 && xlo) || (DY > 0 && ylo) || (DY < 0 && yhi) || (DZ > 0 && zlo) || (DZ < 0 && zhi);
+      float& va = B ? g[a].y : g[a].x;
+      float& vb = B ? g[b].y : g[b].x;
+      if (((Lk >> b) & 1u) && !bwd) va = S::raw_ld(sP, ln);
+      if (((Lk >> a) & 1u) && !fwd) vb = S::raw_ld(sQ, ln + offs<DX, DY, DZ>(G, w));
+    });
+  };
+  if (fluidA && (flA & FLAG_SOLID_LINK)) solid_fix(x, IC<0>{});
+  if (fluidB && (flB & FLAG_SOLID_LINK)) solid_fix(x + 1, IC<1>{});
+  // open x faces: the populations entering through them are rebuilt
+  if (OPEN && ((flA | flB) & FLAG_OPEN)) {
+    if (flA & FLAG_OPEN) {
+      auto at = [&](int i) -> float& { return g[i].x; };
+      if (x == 0) zou_he<1>(p, S::SC, S::INV, at);
+      else zou_he<-1>(p, S::SC, S::INV, at);
+    }
+    if (flB & FLAG_OPEN) zou_he<-1>(p, S::SC, S::INV, [&](int i) -> float& { return g[i].y; });
+  }
+
+  float2 r2, ux2, uy2, uz2;
+  collide_t<Ops2, COLL, SGS, FORCE, PREC>(p, CloNet<SGS>{}, g, r2, ux2, uy2, uz2);
+
+  if (WRITE_MOMENTS && q.active && y < G.ny) {
+    const uint32_t N = (uint32_t)G.n;
+    auto put = [&](float* dst, float a, float b) {
+      if (!(G.nx & 1)) {
+        *reinterpret_cast<float2*>(dst) = make_float2(a, b);
+      } else {  // odd rows start at odd offsets
+        dst[0] = a;
+        if (x + 1 < G.nx) dst[1] = b;
+      }
+    };
+    put(rho_o + nid, fluidA ? r2.x : 0.f, fluidB ? r2.y : 0.f);
+    put(u_o + nid, fluidA ? ux2.x : 0.f, fluidB ? ux2.y : 0.f);
+    put(u_o + (size_t)N + nid, fluidA ? uy2.x : 0.f, fluidB ? uy2.y : 0.f);
+    put(u_o + 2 * (size_t)N + nid, fluidA ? uz2.x : 0.f, fluidB ? uz2.y : 0.f);
+    const bool badA = fluidA && (!(r2.x > 0.f) || !isfinite(r2.x) || !isfinite(ux2.x) || !isfinite(uy2.x) ||
+                                 !isfinite(uz2.x));
+    const bool badB = fluidB && (!(r2.y > 0.f) || !isfinite(r2.y) || !isfinite(ux2.y) || !isfinite(uy2.y) ||
+                                 !isfinite(uz2.y));
+    if (badA || badB) atomicOr(status, 1u);
+  }
+
+  // Solid nodes' slots hold their neighbours' bounce-back values and stay as
+  // they are.  A warp whose pairs are whole (both nodes fluid, or neither) stores
+  // pairs; else node by node, in two branches.
+  const bool both = fluidA && fluidB, none = !fluidA && !fluidB;
+  if (__all_sync(FULL, both || none)) {
+    if (both) {
+      auto put2 = [&](int region, float a, float b) { V2::st(el(region, q.xo), 0, a, b); };
+      put2(0, g[0].x, g[0].y);
+      static_for<0, 9>([&](auto PI) {
+        constexpr int pi = decltype(PI)::value;
+        constexpr int a = pair_a(pi), b = pair_b(pi);
+        put2(1 + 2 * pi, g[b].x, g[b].y);  // f*_b -> X
+        if constexpr (cx(a) == 0) {
+          put2(2 + 2 * pi, g[a].x, g[a].y);  // f*_a -> Y
+        } else {
+          S::raw_st(el(2 + 2 * pi, q.wA), 0, g[a].x);
+          S::raw_st(el(2 + 2 * pi, q.wB), 0, g[a].y);
+        }
+      });
+    }
+  } else {
+    auto put1 = [&](auto sel) {
+      constexpr bool B = decltype(sel)::value != 0;
+      auto at = [&](int i) { return B ? g[i].y : g[i].x; };
+      S::raw_st(el(0, q.xo), B, at(0));
+      static_for<0, 9>([&](auto PI) {
+        constexpr int pi = decltype(PI)::value;
+        constexpr int a = pair_a(pi), b = pair_b(pi);
+        S::raw_st(el(1 + 2 * pi, q.xo), B, at(b));
+        if constexpr (cx(a) == 0) S::raw_st(el(2 + 2 * pi, q.xo), B, at(a));
+        else S::raw_st(el(2 + 2 * pi, B ? q.wB : q.wA), 0, at(a));
+      });
+    };
+    if (fluidA) put1(IC<0>{});
+    if (fluidB) put1(IC<1>{});
+  }
+}
+
+// Flag bytes of a thread's two nodes; nodes that do not exist read as solid.
+__device__ __forceinline__ uint32_t row_flags(const PhysGeom& G, const uint8_t* __restrict__ flags,
+                                              const RowPair& q, int y, int z) {
+  if (!q.active || y >= G.ny) return 0x0101u;
+  const uint32_t nid = (uint32_t)q.x + (uint32_t)G.nx * ((uint32_t)y + (uint32_t)G.ny * (uint32_t)z);
+  if (!(G.nx & 1)) return *reinterpret_cast<const uint16_t*>(flags + nid);
+  const uint32_t b = q.x + 1 < G.nx ? flags[nid + 1] : (uint32_t)FLAG_SOLID;
+  return flags[nid] | b << 8;
+}
+
+template <int PREC, int COLL, int SGS, bool FORCE, bool WRITE_MOMENTS, bool OPEN>
+__global__ void __launch_bounds__(ROWS_THREADS, rows_blocks<PREC, SGS>())
+    k_phys_rows(const __grid_constant__ PhysParams p, RowTiles rt, void* __restrict__ pop_v,
+                const uint8_t* __restrict__ flags, const uint32_t* __restrict__ links,
+                float* __restrict__ rho_o, float* __restrict__ u_o, unsigned* __restrict__ status, int P) {
+  extern __shared__ __align__(128) uint8_t sm[];
+  __shared__ __align__(8) uint64_t bars[2 * ROWS_MAXST];
+  __shared__ uint32_t s_abort;
+  const int cons_warps = (rt.R * rt.tpr + 31) >> 5;  // warps that have nodes
+  const uint32_t full0 = smem_addr(bars), done0 = full0 + 8 * ROWS_MAXST;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < rt.stages; ++s) {
+      // the service warps' bytes, and their lanes' cp.async beside x faces
+      mbar_init(full0 + 8 * s, p.g.per[0] ? ROWS_SERV : ROWS_SERV * 33);
+      mbar_init(done0 + 8 * s, (uint32_t)cons_warps);
+    }
+    s_abort = 0u;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncthreads();
+  const int warp = __shfl_sync(FULL, (int)(threadIdx.x >> 5), 0);  // uniform to the compiler
+  if (warp < ROWS_SERV) {
+    if constexpr (rows_blocks<PREC, SGS>() > 1) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(ROWS_REGS_SERV));
+    rows_service<PREC>(p.g, rt, pop_v, P, warp, smem_addr(sm), full0, done0, &s_abort, status);
+    return;
+  }
+  if constexpr (rows_blocks<PREC, SGS>() > 1) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(ROWS_REGS_CONS));
+  if (warp - ROWS_SERV >= cons_warps) return;
+  const PhysGeom& G = p.g;
+  const RowPair q = row_pair<PREC>(G, rt.R, rt.tpr, (int)threadIdx.x - 32 * ROWS_SERV);
+  const uint32_t stride = gridDim.x;
+  uint32_t s = 0, ph = 0;
+  RowWalk w;
+  w.start(blockIdx.x, stride, rt.tiles_y);
+  int y = w.ty * rt.R + q.row, z = w.z;
+  uint32_t fl = blockIdx.x < rt.ntiles ? row_flags(G, flags, q, y, z) : 0x0101u;
+  for (uint32_t t = blockIdx.x; t < rt.ntiles; t += stride) {
+    const int yc = y, zc = z;
+    const uint32_t flc = fl;
+    if (t + stride < rt.ntiles) {  // the next tile's flags, used one tile later
+      w.next(rt.tiles_y);
+      y = w.ty * rt.R + q.row;
+      z = w.z;
+      fl = row_flags(G, flags, q, y, z);
+    }
+    if (!__all_sync(FULL, mbar_wait(full0 + 8 * s, ph, &s_abort))) {
+      if ((threadIdx.x & 31) == 0) {
+        *reinterpret_cast<volatile uint32_t*>(&s_abort) = 1u;
+        atomicOr(status, 4u);
+      }
+      return;
+    }
+    row_pair_step<PREC, COLL, SGS, FORCE, WRITE_MOMENTS, OPEN>(p, sm + s * rows_stage<PREC>(), q, pop_v, links, rho_o, u_o,
+                                                         status, yc, zc, flc, P);
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0) mbar_arrive(done0 + 8 * s);
+    if (++s == (uint32_t)rt.stages) {
+      s = 0;
+      ph ^= 1u;
+    }
+  }
+}
+
+// Tiles of a grid; R = 0 when a row does not fit.
+inline RowTiles row_tiles(const PhysGeom& G) {
+  RowTiles rt{};
+  if (G.nx < 4 || G.px > ROWS_CAP) return rt;
+  rt.tpr = (G.nx + 1) / 2;
+  if (rt.tpr > ROWS_CONS) return rt;
+  int R = ROWS_CAP / G.px;
+  if (R > ROWS_CONS / rt.tpr) R = ROWS_CONS / rt.tpr;
+  if (R > ROWS_MAXR) R = ROWS_MAXR;
+  if (R > G.ny) R = G.ny;
+  rt.R = R;
+  rt.tiles_y = (G.ny + R - 1) / R;
+  rt.ntiles = (uint32_t)rt.tiles_y * (uint32_t)G.nz;
+  rt.stages = ROWS_MAXST;
+  return rt;
+}
+
+// fp32 stages (45 KB) leave room for one block of five an SM or two of two.
+// Deep prefetch wins where the store streams from HBM (channel 512x128x128 41.6
+// against 38.6 GLUPS, cavity 160^3 37.6 against 34.4); where it stays in the
+// 126 MB L2, twice the consumer warps do (101^3 38.8 against 31.2, 161x97x75
+// with Smagorinsky 33.7 against 27.9, 96^3 38.2 against 29.8).
+inline bool rows_deep(const PhysGeom& G) { return 76.0 * (double)G.slot_stride > 120e6; }
+
+template <int PREC, int COLL, int SGS, bool FORCE, bool WM, bool OPEN>
+cudaError_t launch_row_tiles(const Ctx& c, int P, cudaStream_t s) {
+  RowTiles rt = row_tiles(c.pp.g);
+  const bool deep = PREC == LBM_PREC_F32 && (SGS || rows_deep(c.pp.g));
+  if (PREC == LBM_PREC_F32 && !deep) rt.stages = 2;
+  const size_t smem = (size_t)rt.stages * rows_stage<PREC>();
+  auto* fn = &k_phys_rows<PREC, COLL, SGS, FORCE, WM, OPEN>;
+  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  const uint32_t most = 148u * (deep ? 1 : rows_blocks<PREC, SGS>());
+  const dim3 grd(rt.ntiles < most ? rt.ntiles : most);
+  fn<<<grd, ROWS_THREADS, smem, s>>>(c.pp, rt, c.pop, c.flags, c.links, c.rho, c.u, c.status, P);
+  return cudaGetLastError();
+}
+
+template <int PREC, int COLL, int SGS, bool FORCE>
+cudaError_t rows_wm(const Ctx& c, int P, bool wm, cudaStream_t s) {
+  if (c.pp.any_open)
+    return wm ? launch_row_tiles<PREC, COLL, SGS, FORCE, true, true>(c, P, s)
+              : launch_row_tiles<PREC, COLL, SGS, FORCE, false, true>(c, P, s);
+  return wm ? launch_row_tiles<PREC, COLL, SGS, FORCE, true, false>(c, P, s)
+            : launch_row_tiles<PREC, COLL, SGS, FORCE, false, false>(c, P, s);
+}
+template <int PREC, int COLL>
+cudaError_t rows_coll(const Ctx& c, int P, bool wm, cudaStream_t s) {
+  const bool force = c.pp.accel[0] != 0.f || c.pp.accel[1] != 0.f || c.pp.accel[2] != 0.f;
+  if (c.pp.smag_cs > 0.f)
+    return force ? rows_wm<PREC, COLL, 1, true>(c, P, wm, s) : rows_wm<PREC, COLL, 1, false>(c, P, wm, s);
+  return force ? rows_wm<PREC, COLL, 0, true>(c, P, wm, s) : rows_wm<PREC, COLL, 0, false>(c, P, wm, s);
+}
+
+}  // namespace
+}  // namespace lbm
+
+#define LBM_DEFINE_PHYS_ROWS(NAME, PREC)                                            \
+  namespace lbm {                                                                   \
+  cudaError_t NAME(const Ctx& c, int parity, bool write_moments, cudaStream_t s) {  \
+    return c.d.collision == LBM_COLL_TRT                                            \
+               ? rows_coll<PREC, LBM_COLL_TRT>(c, parity, write_moments, s)         \
+               : rows_coll<PREC, LBM_COLL_BGK>(c, parity, write_moments, s);        \
+  }                                                                                 \
+  }

@@ -51,7 +51,7 @@ template <> struct Store<LBM_PREC_BF16S> {
 
 namespace {
 
-__device__ __forceinline__ size_t lin(const PhysGeom& g, int x, int y, int z) {
+__host__ __device__ __forceinline__ size_t lin(const PhysGeom& g, int x, int y, int z) {
   return (size_t)x + (size_t)g.px * ((size_t)(y + g.gy) + (size_t)g.py * (size_t)(z + g.gz));
 }
 
@@ -81,7 +81,7 @@ __device__ __forceinline__ float wall_term(const PhysParams& p, int x, int y, in
   else if (!g.per[0] && (tx < 0 || tx >= g.nx)) face = tx < 0 ? LBM_FACE_XM : LBM_FACE_XP;
   if (face < 0) return 0.0f;
   const float cu = cx(J) * p.wall[face][0] + cy(J) * p.wall[face][1] + cz(J) * p.wall[face][2];
-  return 6.0f * wf(J) * cu;
+  return __fmul_rn(6.0f * wf(J), cu);  // never contracted into the sum that takes it
 }
 
 // Open x face (Zou & He 1997; D3Q19 form of Hecht & Harting 2010): the five

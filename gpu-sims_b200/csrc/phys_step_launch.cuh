@@ -2,7 +2,7 @@
 // precision by phys_step_{f32,f16,bf16}.cu and, for the learned closure, by
 // phys_step_clo_{f32,f16,bf16}.cu (split so the six compile in parallel).  The kernels wrap step_row / step_row2 (phys_step.cuh).
 #pragma once
-#include "phys_step.cuh"
+#include "phys_rows.cuh"
 
 namespace lbm {
 namespace {
@@ -286,6 +286,32 @@ inline bool use_quads(const Ctx& c) {
   if (c.closure || c.pp.any_open || nx % 4) return false;
   return c.step_variant == 4 || (c.step_variant == 0 && step_quads(nx));
 }
+// Row tiles (phys_rows.cuh) by default where rows fill their blocks and the
+// grid has enough tiles to fill the persistent blocks (148 or 296) several
+// times; else the row kernels' small blocks win.  The lines, measured on B200
+// (row tiles / row kernels, GLUPS):
+//  * rows below 66 nodes waste padding and tiles: 64^3 22.8 / 30.2 (fp16), 56 x
+//    56 x 200 29.5 / 36.2 (fp32), 57 x 57 x 200 26.0 / 31.0 (fp16);
+//  * nodes per 512-node tile: fp32 144^3 (0.84) 36.6 / 31.9, 200 x 97 x 120 (0.78)
+//    34.7 / 32.4, 385 x 97 x 120 (0.75) 32.9 / 31.4, 180 x 97 x 120 (0.70) 32.2 / 33.8,
+//    257 x 97 x 120 (0.50) 24.7 / 30.2; fp16 200 x 97 x 120 53.3 / 43.0, 192^3 (0.75)
+//    48.8 / 58.4, 320 x 97 x 120 (0.63) 54.9 / 56.5; odd rows, which only the one-node
+//    kernel takes otherwise, pay in 2-byte storage at any fill (257 43.3 / 35.1);
+//  * rows that leave the row kernels' 64-wide warps ragged: fp16 72^3 (792 tiles)
+//    27.2 / 23.4, fp32 72^3 24.2 / 24.2, 80^3 (1,120) 29.7 / 28.4;
+//  * rows of whole warps: fp16 128^3 (4,096) 56.1 / 55.6, 256 x 256 x 8 (1,024)
+//    45.1 / 51.9; fp32 256 x 128 x 128 (8,192) 37.8 / 38.3, 512 x 128 x 128 (16,384)
+//    41.2 / 39.4, 256^3 (32,768) 42.5 / 41.6.
+inline bool use_row_tiles(const Ctx& c) {
+  if (c.step_variant != 0 || c.closure) return false;
+  const int nx = c.pp.g.nx;
+  const RowTiles rt = row_tiles(c.pp.g);
+  if (rt.R == 0 || nx < 66) return false;
+  const bool odd = nx % 2 != 0, whole = !odd && 20 * ((nx + 63) / 64 * 64) <= 23 * nx;
+  const int fill = 100 * rt.R * nx / 512;  // per cent of a tile
+  if (c.d.precision == LBM_PREC_F32) return fill >= 74 && rt.ntiles >= (whole ? 12000u : 1000u);
+  return (odd || fill >= 76) && rt.ntiles >= (whole ? 4000u : 700u);
+}
 inline bool use_pairs(const Ctx& c) {
   const int nx = c.pp.g.nx;
   if (nx % 2 || c.step_variant == 1 || c.step_variant == 8) return false;
@@ -296,8 +322,10 @@ template <int PREC, int COLL, int SGS, bool FORCE>
 cudaError_t launch_rows(const Ctx& c, int P, bool wm, cudaStream_t s) {
   const PhysGeom& G = c.pp.g;
   const CloNet<SGS> net = net_of<SGS>(c);
-  const dim3 blk(32, STEP_BY, 1);
   if constexpr (SGS != 2) {
+    if (use_row_tiles(c))
+      return PREC == LBM_PREC_F32 ? phys_rows_f32(c, P, wm, s)
+             : PREC == LBM_PREC_F16S ? phys_rows_f16(c, P, wm, s) : phys_rows_bf16(c, P, wm, s);
     if (use_quads(c)) {
       constexpr int R4 = LBM_STEP4_ROWS;
       const dim3 grd((G.nx + 127) / 128, (G.ny + R4 - 1) / R4, G.nz), blk4(32, R4, 1);
@@ -345,7 +373,7 @@ cudaError_t launch_rows(const Ctx& c, int P, bool wm, cudaStream_t s) {
 template <int PREC, int COLL, int SGS, bool FORCE>
 cudaError_t launch_step(const Ctx& c, int P, bool wm, cudaStream_t s) {
   const cudaError_t e = launch_rows<PREC, COLL, SGS, FORCE>(c, P, wm, s);
-  if (e != cudaSuccess || !c.pp.any_open) return e;
+  if (e != cudaSuccess || !c.pp.any_open || (SGS != 2 && use_row_tiles(c))) return e;
   const CloNet<SGS> net = net_of<SGS>(c);
   const dim3 grd((c.pp.g.ny * c.pp.g.nz + 127) / 128, 2, 1);
 #define LBM_FACE_LAUNCH(WM, PAR)                                          \

@@ -194,7 +194,8 @@ LBM_API int lbm_init_from_moments(lbm_ctx* ctx, const float* rho, const void* u,
  * The moments of the last step are written for readback. */
 LBM_API int lbm_step(lbm_ctx* ctx, int nsteps);
 
-/* Physics mode: kernel variant of the step.  0 = automatic (two nodes per
+/* Physics mode: kernel variant of the step.  0 = automatic (rows streamed
+ * through shared memory where the grid has enough of them; else two nodes per
  * thread when nx is even and the rows fill 64-wide warps, else one); 1, 2 or
  * 4 nodes per thread (4: nx % 4 == 0; one 16-byte access per slot quad for
  * fp32 storage, 8-byte for fp16/bf16); 8 = one node per
