@@ -41,7 +41,7 @@ namespace lbm {
 namespace {
 
 constexpr int ROWS_CAP = 576;    // elements of a tile in one slot array
-constexpr int ROWS_MAXR = 16;    // rows of a tile
+constexpr int ROWS_MAXR = 12;    // rows of a tile
 constexpr int ROWS_CONS = 256;   // consumer threads
 constexpr int ROWS_SERV = 4;     // service warps, which issue the copies
 constexpr int ROWS_MAXST = 5;
@@ -71,8 +71,8 @@ constexpr int rows_blocks() {
 }
 // Two blocks of 12 warps leave 80 registers a thread at launch (384 * 80 =
 // 30,720 a block); the service warpgroup hands its share on:
-// 128 * 40 + 256 * 96 = 29,696.
-constexpr int ROWS_REGS_SERV = 40, ROWS_REGS_CONS = 96;
+// 128 * 48 + 256 * 96 = 30,720.
+constexpr int ROWS_REGS_SERV = 48, ROWS_REGS_CONS = 96;
 static_assert(128 * ROWS_REGS_SERV + ROWS_CONS * ROWS_REGS_CONS <= ROWS_THREADS * 80, "registers of a block");
 
 struct RowTiles {
@@ -252,46 +252,88 @@ __host__ __device__ __forceinline__ ptrdiff_t side_offset(const PhysGeom& G, int
          (ptrdiff_t)dz * (ptrdiff_t)G.pxy + (EB == 2 ? G.nx & ~1 : G.nx);
 }
 
-// A service warp.  One lane issues the copies of its arrays: their operands are
-// then uniform over the warp, and each costs a handful of instructions.
+// The barriers of a block's stages, and its abort mark.
+struct RowBars {
+  uint32_t full, done;  // shared addresses: rows landed, nodes collided
+  volatile uint32_t* abort;
+  unsigned* status;
+  __device__ __forceinline__ void give_up() const {
+    if ((threadIdx.x & 31) == 0) {
+      *abort = 1u;
+      atomicOr(status, 4u);
+    }
+  }
+};
+// A stage index and its phase parity, in tile order.
+struct RowStage {
+  uint32_t s = 0, ph = 0;
+  __device__ __forceinline__ void next(uint32_t stages) {
+    if (++s == stages) {
+      s = 0;
+      ph ^= 1u;
+    }
+  }
+};
+
+__device__ __forceinline__ bool inner_tile(const PhysGeom& G, int y0, int z, int rows) {
+  return y0 > 0 && y0 + rows < G.ny && z > 0 && z < G.nz - 1;
+}
+constexpr int ROWS_NA = (Q + ROWS_SERV - 1) / ROWS_SERV;  // arrays of a service warp: part, part + ROWS_SERV, ...
+constexpr uint64_t ROWS_MOST_BYTES = 1ull << 36;          // of a store (32-bit offsets of 16 bytes, below)
+
+// The tiles of one domain in a block's walk: `count` of them from tile `first`
+// on, `stride` apart.
+struct RowSeg {
+  RowTiles rt;
+  uint32_t first, stride, count;
+};
+
+// A service warp's part of a segment: loads ahead of the collision and writes
+// back behind it.  One lane issues the copies of the warp's arrays: their
+// operands are then uniform over the warp, and each costs a handful of
+// instructions.  The segment's rows have left the stages when it ends, so the
+// next one (another domain) starts from empty stages.  False when a wait gave
+// up.
 template <int PREC>
-__device__ __forceinline__ void rows_service(const PhysGeom& G, const RowTiles& rt, void* pop, int P, int part,
-                                              uint32_t stage0, uint32_t full0, uint32_t done0,
-                                              volatile uint32_t* abort, unsigned* status) {
+__device__ __forceinline__ bool rows_service(const PhysGeom& G, const RowSeg& sg, void* pop, int P, int part,
+                                             uint32_t stage0, const RowBars& B, uint32_t stages, RowStage& st_) {
   using T = typename Store<PREC>::T;
   constexpr uint32_t EB = sizeof(T);
-  constexpr int NA = (Q + ROWS_SERV - 1) / ROWS_SERV;  // arrays of a service warp: part, part + ROWS_SERV, ...
   const int lane = threadIdx.x & 31;
   char* base = reinterpret_cast<char*>(pop);
   const uint32_t row_bytes = (uint32_t)G.px * EB;
-  const uint32_t n = rt.ntiles <= blockIdx.x ? 0u : (rt.ntiles - blockIdx.x + gridDim.x - 1) / gridDim.x;
-  const uint32_t stages = (uint32_t)rt.stages;
   const uint32_t arrays = (uint32_t)((Q + ROWS_SERV - 1 - part) / ROWS_SERV);
-  ptrdiff_t off[NA];
+  // The warp's arrays away from the y and z faces, in 16-byte units from a
+  // tile's first element in array 0 (never negative: an array's rows lie beyond
+  // the arrays before it).
+  uint32_t off[ROWS_NA];
 #pragma unroll
-  for (int i = 0; i < NA; ++i) off[i] = array_offset(G, min(part + ROWS_SERV * i, Q - 1), P) * (ptrdiff_t)EB;
-  const uint32_t region0 = (uint32_t)part * rows_region<PREC>();
+  for (int i = 0; i < ROWS_NA; ++i) {
+    off[i] = (uint32_t)((uint64_t)array_offset(G, min(part + ROWS_SERV * i, Q - 1), P) * EB / 16);
+    asm volatile("" : "+r"(off[i]));  // not recomputed, nor kept in 64 bits
+  }
   // this lane's x-face value of a row: where it lies from the row's first
   // element in array 0 (tiles away from the y and z faces), and its place
   const int side_row = lane < 30 ? lane / 10 : ROWS_MAXR, side_e = lane % 10;
   uint32_t side_dst;
   const ptrdiff_t side_src = side_offset<PREC>(G, P, side_e, side_dst) * (ptrdiff_t)EB;
-  auto inner = [&](int y0, int z, int rows) { return y0 > 0 && y0 + rows < G.ny && z > 0 && z < G.nz - 1; };
   RowWalk wl, ws;  // of the loads and of the stores
-  wl.start(blockIdx.x, gridDim.x, rt.tiles_y);
+  wl.start(sg.first, sg.stride, sg.rt.tiles_y);
   ws = wl;
   auto load = [&](uint32_t s) {
-    const int z = wl.z, y0 = wl.ty * rt.R, rows = min(rt.R, G.ny - y0);
-    const uint32_t st = stage0 + s * rows_stage<PREC>(), bar = full0 + 8 * s;
+    const int z = wl.z, y0 = wl.ty * sg.rt.R, rows = min(sg.rt.R, G.ny - y0);
+    const uint32_t st = stage0 + s * rows_stage<PREC>(), bar = B.full + 8 * s;
+    const char* at = base + lin(G, 0, y0, z) * EB;
+    const bool in = inner_tile(G, y0, z, rows);
     if (lane == 0) {
-      char* at = base + lin(G, 0, y0, z) * EB;
       const uint32_t bytes = (uint32_t)rows * row_bytes;
       mbar_arrive_tx(bar, bytes * arrays);
-      if (inner(y0, z, rows)) {
+      if (in) {
 #pragma unroll
-        for (int i = 0; i < NA; ++i)
-          if (part + ROWS_SERV * i < Q)
-            bulk_load(st + region0 + ROWS_SERV * i * rows_region<PREC>(), at + off[i], bytes, bar);
+        for (int i = 0; i < ROWS_NA; ++i) {
+          const int k = part + ROWS_SERV * i;
+          if (k < Q) bulk_load(st + k * rows_region<PREC>(), at + (uint64_t)off[i] * 16, bytes, bar);
+        }
       } else {
 #pragma unroll 1
         for (int k = part; k < Q; k += ROWS_SERV)
@@ -304,40 +346,41 @@ __device__ __forceinline__ void rows_service(const PhysGeom& G, const RowTiles& 
     __syncwarp();
     if (!G.per[0]) {
       // ten lanes a row, three rows a warp
-      const char* at = base + lin(G, 0, y0, z) * EB + side_src;
-      const bool in = inner(y0, z, rows);
       for (int r = 3 * part + side_row; r < rows; r += 3 * ROWS_SERV) {
-        const char* src = at + (uint32_t)r * row_bytes;
+        const char* src = at + side_src + (uint32_t)r * row_bytes;
         uint32_t o = side_dst + 4u * (uint32_t)r;
         if (!in) src = reinterpret_cast<const char*>(row_side<PREC>(G, pop, P, 10 * r + side_e, y0, z, o));
         asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(st + o), "l"(src) : "memory");
       }
-      asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
     }
-    wl.next(rt.tiles_y);
+    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
+    wl.next(sg.rt.tiles_y);
   };
-  const uint32_t ahead = min(stages, n);
-  #pragma unroll 1
-  for (uint32_t j = 0; j < ahead; ++j) load(j);
-  uint32_t loaded = ahead, s = 0, ph = 0, prev = 0;
-  for (uint32_t j = 0; j < n; ++j) {
-    const bool ok = mbar_wait(done0 + 8 * s, ph, abort);
-    if (!__all_sync(FULL, ok)) {
-      if (lane == 0) {
-        *abort = 1u;
-        atomicOr(status, 4u);
-      }
+  uint32_t loaded = 0, sl = st_.s;
+#pragma unroll 1
+  for (; loaded < min(stages, sg.count); ++loaded) {
+    load(sl);
+    if (++sl == stages) sl = 0;
+  }
+  uint32_t prev = 0;
+  bool ok = true;
+#pragma unroll 1
+  for (uint32_t j = 0; j < sg.count; ++j) {
+    ok = __all_sync(FULL, mbar_wait(B.done + 8 * st_.s, st_.ph, B.abort));
+    if (!ok) {
+      B.give_up();
       break;
     }
-    const int z = ws.z, y0 = ws.ty * rt.R, rows = min(rt.R, G.ny - y0);
     if (lane == 0) {
-      const uint32_t st = stage0 + s * rows_stage<PREC>();
+      const int z = ws.z, y0 = ws.ty * sg.rt.R, rows = min(sg.rt.R, G.ny - y0);
+      const uint32_t st = stage0 + st_.s * rows_stage<PREC>();
       char* at = base + lin(G, 0, y0, z) * EB;
-      if (inner(y0, z, rows)) {
+      if (inner_tile(G, y0, z, rows)) {
 #pragma unroll
-        for (int i = 0; i < NA; ++i)
-          if (part + ROWS_SERV * i < Q)
-            bulk_store(at + off[i], st + region0 + ROWS_SERV * i * rows_region<PREC>(), (uint32_t)rows * row_bytes);
+        for (int i = 0; i < ROWS_NA; ++i) {
+          const int k = part + ROWS_SERV * i;
+          if (k < Q) bulk_store(at + (uint64_t)off[i] * 16, st + k * rows_region<PREC>(), (uint32_t)rows * row_bytes);
+        }
       } else {
 #pragma unroll 1
         for (int k = part; k < Q; k += ROWS_SERV)
@@ -353,29 +396,31 @@ __device__ __forceinline__ void rows_service(const PhysGeom& G, const RowTiles& 
       else asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
     }
     __syncwarp();
-    ws.next(rt.tiles_y);
-    if (stages <= 2) prev = s;
-    if ((j > 0 || stages <= 2) && loaded < n) {
+    ws.next(sg.rt.tiles_y);
+    if (stages <= 2) prev = st_.s;
+    if ((j > 0 || stages <= 2) && loaded < sg.count) {
       load(prev);
       ++loaded;
     }
-    prev = s;
-    if (++s == stages) {
-      s = 0;
-      ph ^= 1u;
+    prev = st_.s;
+    st_.next(stages);
+  }
+  if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+  __syncwarp();
+  if (!ok) {
+    // leave no load in flight: each stage's current phase, if it has loads
+    for (uint32_t k = 0; k < stages && k < loaded; ++k) {
+      for (uint32_t i = 0; i < ROWS_WAIT_LIMIT; ++i)
+        if (mbar_try(B.full + 8 * st_.s, st_.ph)) break;
+      st_.next(stages);
     }
   }
-  if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
-  if (*abort) {
-    // leave no copy in flight: the loads that no consumer waited for
-    for (uint32_t j = loaded > stages ? loaded - stages : 0u; j < loaded; ++j)
-      for (uint32_t i = 0; i < ROWS_WAIT_LIMIT; ++i)
-        if (mbar_try(full0 + 8 * (j % stages), (j / stages) & 1u)) break;
-  }
+  return ok;
 }
 
 // One pair of nodes' step on a landed tile: stream from, and collide into, the
 // stage at st.
+// (cp holds what the collision reads, p everything.)
 struct RowPair {
   int row, x;              // row within the tile, x of node A
   bool active;             // the thread has a pair
@@ -411,7 +456,8 @@ __host__ __device__ __forceinline__ RowPair row_pair(const PhysGeom& G, int R, i
 }
 
 template <int PREC, int COLL, int SGS, bool FORCE, bool WRITE_MOMENTS, bool OPEN>
-__device__ __forceinline__ void row_pair_step(const PhysParams& p, uint8_t* __restrict__ st, const RowPair& q,
+__device__ __forceinline__ void row_pair_step(const PhysParams& p, const PhysParams& cp, const PhysGeom& G, int moving,
+                                              uint8_t* __restrict__ st, const RowPair& q,
                                               void* __restrict__ pop_v, const uint32_t* __restrict__ links,
                                               float* __restrict__ rho_o, float* __restrict__ u_o,
                                               unsigned* __restrict__ status, int y, int z, uint32_t fl2, int P) {
@@ -419,7 +465,6 @@ __device__ __forceinline__ void row_pair_step(const PhysParams& p, uint8_t* __re
   using V2 = Vec2<PREC>;
   using T = typename S::T;
   constexpr int REG = rows_region<PREC>();
-  const PhysGeom& G = p.g;
   const int x = q.x;
   auto el = [&](int region, uint32_t off) -> T* { return reinterpret_cast<T*>(st + region * REG + off); };
   auto one = [&](int region, uint32_t off) { return S::raw_ld(el(region, off), 0); };
@@ -443,7 +488,7 @@ __device__ __forceinline__ void row_pair_step(const PhysParams& p, uint8_t* __re
   const uint32_t nid = (uint32_t)x + (uint32_t)G.nx * ((uint32_t)y + (uint32_t)G.ny * (uint32_t)z);
   const uint32_t flA = fl2 & 0xffu, flB = fl2 >> 8;
   const bool fluidA = !(flA & FLAG_SOLID), fluidB = !(flB & FLAG_SOLID);
-  if (p.any_moving_wall && near_moving(p, x, x + 1 < G.nx ? x + 1 : x, y, z)) {
+  if (moving && near_moving(moving, G, x, x + 1 < G.nx ? x + 1 : x, y, z)) {
     auto faces = [&](int xx, auto sel) {
       constexpr bool B = decltype(sel)::value != 0;
       const bool xlo = !G.per[0] && xx == 0, xhi = !G.per[0] && xx == G.nx - 1;
@@ -502,7 +547,7 @@ __device__ __forceinline__ void row_pair_step(const PhysParams& p, uint8_t* __re
   }
 
   float2 r2, ux2, uy2, uz2;
-  collide_t<Ops2, COLL, SGS, FORCE, PREC>(p, CloNet<SGS>{}, g, r2, ux2, uy2, uz2);
+  collide_t<Ops2, COLL, SGS, FORCE, PREC>(cp, CloNet<SGS>{}, g, r2, ux2, uy2, uz2);
 
   if (WRITE_MOMENTS && q.active && y < G.ny) {
     const uint32_t N = (uint32_t)G.n;
@@ -573,82 +618,116 @@ __device__ __forceinline__ uint32_t row_flags(const PhysGeom& G, const uint8_t* 
   return flags[nid] | b << 8;
 }
 
+// What a block needs of the domain whose tiles it walks.
+struct RowDomain {
+  void* pop;
+  const uint8_t* flags;
+  const uint32_t* links;
+  float *rho, *u;
+};
+
+// A consumer thread's part of a segment.  False when a wait gave up.
 template <int PREC, int COLL, int SGS, bool FORCE, bool WRITE_MOMENTS, bool OPEN>
-__global__ void __launch_bounds__(ROWS_THREADS, rows_blocks<PREC, SGS>())
-    k_phys_rows(const __grid_constant__ PhysParams p, RowTiles rt, void* __restrict__ pop_v,
-                const uint8_t* __restrict__ flags, const uint32_t* __restrict__ links,
-                float* __restrict__ rho_o, float* __restrict__ u_o, unsigned* __restrict__ status, int P) {
+__device__ __forceinline__ bool rows_consume(const PhysParams& p, const PhysParams& cp, const PhysGeom& G, int moving,
+                                             const RowSeg& sg, const RowDomain& D, uint8_t* sm, int tid, int P,
+                                             const RowBars& B, uint32_t stages, RowStage& st_) {
+  const RowPair q = row_pair<PREC>(G, sg.rt.R, sg.rt.tpr, tid);
+  RowWalk w;
+  w.start(sg.first, sg.stride, sg.rt.tiles_y);
+  int y = w.ty * sg.rt.R + q.row, z = w.z;
+  uint32_t fl = row_flags(G, D.flags, q, y, z);
+  for (uint32_t j = 0; j < sg.count; ++j) {
+    const int yc = y, zc = z;
+    const uint32_t flc = fl;
+    if (j + 1 < sg.count) {  // the next tile's flags, used one tile later
+      w.next(sg.rt.tiles_y);
+      y = w.ty * sg.rt.R + q.row;
+      z = w.z;
+      fl = row_flags(G, D.flags, q, y, z);
+    }
+    if (!__all_sync(FULL, mbar_wait(B.full + 8 * st_.s, st_.ph, B.abort))) {
+      B.give_up();
+      return false;
+    }
+    row_pair_step<PREC, COLL, SGS, FORCE, WRITE_MOMENTS, OPEN>(p, cp, G, moving, sm + st_.s * rows_stage<PREC>(), q,
+                                                               D.pop, D.links, D.rho, D.u, B.status, yc, zc, flc, P);
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0) mbar_arrive(B.done + 8 * st_.s);
+    st_.next(stages);
+  }
+  return true;
+}
+
+// Set-up of a block: barriers, roles and the share of the registers; cons_warps
+// consumer warps take part.  SEGS is
+// called as segs(f) and calls f(p, cp, G, moving, segment, domain) for the
+// block's segments in order until f returns false.
+template <int PREC, int COLL, int SGS, bool FORCE, bool WRITE_MOMENTS, bool OPEN, class SEGS>
+__device__ __forceinline__ void rows_block(uint32_t stages, uint32_t cons_warps, unsigned* status, int P, SEGS&& segs) {
   extern __shared__ __align__(128) uint8_t sm[];
   __shared__ __align__(8) uint64_t bars[2 * ROWS_MAXST];
   __shared__ uint32_t s_abort;
-  const int cons_warps = (rt.R * rt.tpr + 31) >> 5;  // warps that have nodes
-  const uint32_t full0 = smem_addr(bars), done0 = full0 + 8 * ROWS_MAXST;
+  RowBars B;
+  B.full = smem_addr(bars);
+  B.done = B.full + 8 * ROWS_MAXST;
+  B.abort = &s_abort;
+  B.status = status;
   if (threadIdx.x == 0) {
-    for (int s = 0; s < rt.stages; ++s) {
-      // the service warps' bytes, and their lanes' cp.async beside x faces
-      mbar_init(full0 + 8 * s, p.g.per[0] ? ROWS_SERV : ROWS_SERV * 33);
-      mbar_init(done0 + 8 * s, (uint32_t)cons_warps);
+    for (uint32_t s = 0; s < stages; ++s) {
+      mbar_init(B.full + 8 * s, ROWS_SERV * 33);  // the service warps' bytes, and their lanes' cp.async
+      mbar_init(B.done + 8 * s, cons_warps);
     }
     s_abort = 0u;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
   const int warp = __shfl_sync(FULL, (int)(threadIdx.x >> 5), 0);  // uniform to the compiler
+  RowStage st;
   if (warp < ROWS_SERV) {
     if constexpr (rows_blocks<PREC, SGS>() > 1) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(ROWS_REGS_SERV));
-    rows_service<PREC>(p.g, rt, pop_v, P, warp, smem_addr(sm), full0, done0, &s_abort, status);
+    segs([&](const PhysParams&, const PhysParams&, const PhysGeom& G, int, const RowSeg& sg, const RowDomain& D) {
+      return rows_service<PREC>(G, sg, D.pop, P, warp, smem_addr(sm), B, stages, st);
+    });
+    if ((threadIdx.x & 31) == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     return;
   }
   if constexpr (rows_blocks<PREC, SGS>() > 1) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(ROWS_REGS_CONS));
-  if (warp - ROWS_SERV >= cons_warps) return;
-  const PhysGeom& G = p.g;
-  const RowPair q = row_pair<PREC>(G, rt.R, rt.tpr, (int)threadIdx.x - 32 * ROWS_SERV);
-  const uint32_t stride = gridDim.x;
-  uint32_t s = 0, ph = 0;
-  RowWalk w;
-  w.start(blockIdx.x, stride, rt.tiles_y);
-  int y = w.ty * rt.R + q.row, z = w.z;
-  uint32_t fl = blockIdx.x < rt.ntiles ? row_flags(G, flags, q, y, z) : 0x0101u;
-  for (uint32_t t = blockIdx.x; t < rt.ntiles; t += stride) {
-    const int yc = y, zc = z;
-    const uint32_t flc = fl;
-    if (t + stride < rt.ntiles) {  // the next tile's flags, used one tile later
-      w.next(rt.tiles_y);
-      y = w.ty * rt.R + q.row;
-      z = w.z;
-      fl = row_flags(G, flags, q, y, z);
-    }
-    if (!__all_sync(FULL, mbar_wait(full0 + 8 * s, ph, &s_abort))) {
-      if ((threadIdx.x & 31) == 0) {
-        *reinterpret_cast<volatile uint32_t*>(&s_abort) = 1u;
-        atomicOr(status, 4u);
-      }
-      return;
-    }
-    row_pair_step<PREC, COLL, SGS, FORCE, WRITE_MOMENTS, OPEN>(p, sm + s * rows_stage<PREC>(), q, pop_v, links, rho_o, u_o,
-                                                         status, yc, zc, flc, P);
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    __syncwarp();
-    if ((threadIdx.x & 31) == 0) mbar_arrive(done0 + 8 * s);
-    if (++s == (uint32_t)rt.stages) {
-      s = 0;
-      ph ^= 1u;
-    }
-  }
+  if ((uint32_t)(warp - ROWS_SERV) >= cons_warps) return;
+  segs([&](const PhysParams& p, const PhysParams& cp, const PhysGeom& G, int moving, const RowSeg& sg,
+           const RowDomain& D) {
+    return rows_consume<PREC, COLL, SGS, FORCE, WRITE_MOMENTS, OPEN>(p, cp, G, moving, sg, D, sm,
+                                                                           (int)threadIdx.x - 32 * ROWS_SERV, P, B, stages, st);
+  });
+}
+
+// One domain: block b takes tiles b, b + gridDim.x, ...
+template <int PREC, int COLL, int SGS, bool FORCE, bool WRITE_MOMENTS, bool OPEN>
+__global__ void __launch_bounds__(ROWS_THREADS, rows_blocks<PREC, SGS>())
+    k_phys_rows(const __grid_constant__ PhysParams p, RowTiles rt, void* __restrict__ pop_v,
+                const uint8_t* __restrict__ flags, const uint32_t* __restrict__ links,
+                float* __restrict__ rho_o, float* __restrict__ u_o, unsigned* __restrict__ status, int P) {
+  const RowDomain D{pop_v, flags, links, rho_o, u_o};
+  const RowSeg sg{rt, blockIdx.x, gridDim.x,
+                  rt.ntiles <= blockIdx.x ? 0u : (rt.ntiles - blockIdx.x + gridDim.x - 1) / gridDim.x};
+  const uint32_t cons_warps = (uint32_t)(rt.R * rt.tpr + 31) / 32;  // warps that have nodes
+  rows_block<PREC, COLL, SGS, FORCE, WRITE_MOMENTS, OPEN>((uint32_t)rt.stages, cons_warps, status, P, [&](auto&& f) {
+    if (sg.count) f(p, p, p.g, p.any_moving_wall, sg, D);
+  });
 }
 
 // Tiles of a grid; R = 0 when a row does not fit.
 inline RowTiles row_tiles(const PhysGeom& G) {
   RowTiles rt{};
-  if (G.nx < 4 || G.px > ROWS_CAP) return rt;
+  if (G.nx < 4 || G.px > ROWS_CAP || (uint64_t)Q * G.slot_stride * 4 >= ROWS_MOST_BYTES) return rt;
   rt.tpr = (G.nx + 1) / 2;
   if (rt.tpr > ROWS_CONS) return rt;
   int R = ROWS_CAP / G.px;
   if (R > ROWS_CONS / rt.tpr) R = ROWS_CONS / rt.tpr;
   if (R > ROWS_MAXR) R = ROWS_MAXR;
   if (R > G.ny) R = G.ny;
-  rt.R = R;
   rt.tiles_y = (G.ny + R - 1) / R;
+  rt.R = (G.ny + rt.tiles_y - 1) / rt.tiles_y;  // as even as the count allows
   rt.ntiles = (uint32_t)rt.tiles_y * (uint32_t)G.nz;
   rt.stages = ROWS_MAXST;
   return rt;
@@ -659,12 +738,12 @@ inline RowTiles row_tiles(const PhysGeom& G) {
 // against 38.6 GLUPS, cavity 160^3 37.6 against 34.4); where it stays in the
 // 126 MB L2, twice the consumer warps do (101^3 38.8 against 31.2, 161x97x75
 // with Smagorinsky 33.7 against 27.9, 96^3 38.2 against 29.8).
-inline bool rows_deep(const PhysGeom& G) { return 76.0 * (double)G.slot_stride > 120e6; }
+constexpr size_t ROWS_DEEP_BYTES = 120000000;
 
 template <int PREC, int COLL, int SGS, bool FORCE, bool WM, bool OPEN>
 cudaError_t launch_row_tiles(const Ctx& c, int P, cudaStream_t s) {
   RowTiles rt = row_tiles(c.pp.g);
-  const bool deep = PREC == LBM_PREC_F32 && (SGS || rows_deep(c.pp.g));
+  const bool deep = PREC == LBM_PREC_F32 && (SGS || 76 * c.pp.g.slot_stride > ROWS_DEEP_BYTES);
   if (PREC == LBM_PREC_F32 && !deep) rt.stages = 2;
   const size_t smem = (size_t)rt.stages * rows_stage<PREC>();
   auto* fn = &k_phys_rows<PREC, COLL, SGS, FORCE, WM, OPEN>;
