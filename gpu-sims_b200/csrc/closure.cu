@@ -31,6 +31,33 @@ float round_bf16(float v) {
   return r;
 }
 
+void clo_fragments(const float* net, uint32_t* words) {
+  auto bits = [](float v) {  // a bf16 value's upper half
+    uint32_t u;
+    std::memcpy(&u, &v, 4);
+    return u >> 16;
+  };
+  auto w1 = [&](int n, int k) { return k < 30 && k % 10 < CLO_IN ? net[CLO_W1 + n * CLO_IN + k % 10] : 0.0f; };
+  auto w2 = [&](int n, int k) { return net[CLO_W2 + n * CLO_HID + k]; };
+  for (int lane = 0; lane < 32; ++lane) {
+    const int g = lane >> 2, t = lane & 3;
+    for (int s = 0; s < 2; ++s)
+      for (int j = 0; j < 4; ++j)
+        for (int h = 0; h < 2; ++h) {  // rows k and k + 1 of column n
+          const int n = 8 * j + g, k = 16 * s + 8 * h + 2 * t;
+          const size_t at = ((size_t)((2 * s + j / 2) * 32 + lane)) * 4 + 2 * (j % 2) + h;
+          words[at] = bits(w1(n, k)) | bits(w1(n, k + 1)) << 16;
+          words[512 + at] = bits(w2(n, k)) | bits(w2(n, k + 1)) << 16;
+        }
+  }
+  const int src[3] = {CLO_B1, CLO_B2, CLO_W3};
+  for (int v = 0; v < 3; ++v)
+    for (int j = 0; j < 4; ++j)
+      for (int t = 0; t < 4; ++t)
+        for (int e = 0; e < 2; ++e)
+          std::memcpy(&words[1024 + ((2 * v + j / 2) * 4 + t) * 4 + 2 * (j % 2) + e], &net[src[v] + 8 * j + 2 * t + e], 4);
+}
+
 namespace {
 
 // ---------------------------------------------------------------------------

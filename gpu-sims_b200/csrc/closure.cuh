@@ -28,6 +28,7 @@ template <int SGS> struct CloNet {
 };
 template <> struct CloNet<2> {
   float v[CLO_FLOATS];
+  const uint4* frag;  // device: the layers as matrix fragments (clo_fragments)
   __device__ __forceinline__ float operator[](int k) const { return v[k]; }
 };
 
@@ -119,7 +120,7 @@ __device__ __forceinline__ void closure_features(const typename O::F (&P)[6], ty
 }
 
 // Forward pass: standardised inputs -> ReLU(32) -> ReLU(32) -> softplus.
-// w[k] reads parameter k (a CloNet<2> in parameter space, or shared memory).
+// w[k] reads parameter k (shared memory).
 template <class O, class W>
 __device__ __forceinline__ typename O::F closure_mlp(const W& w, const typename O::F (&xr)[CLO_IN]) {
   using F = typename O::F;
@@ -144,6 +145,160 @@ __device__ __forceinline__ typename O::F closure_mlp(const W& w, const typename 
     z = O::fma(O::splat(w[CLO_W3 + i]), O::relu(a), z);
   }
   return O::softplus(z);
+}
+
+// ---------------------------------------------------------------------------
+// The default evaluation in the step kernels: both layers as warp-level matrix
+// products (mma.sync m16n8k16, bf16 in, fp32 accumulators), 32 nodes a warp at a
+// time.  The weights are bf16 values already; every activation enters as the sum
+// of three bf16 numbers (8 + 8 + 8 bits, the whole fp32 significand), so each
+// product is exact and only the fp32 sums round, as on the CUDA cores.
+//
+// Why not tcgen05 here: the layers are 9 x 32 and 32 x 32, so a node's chain is
+// features -> layer -> layer -> r, and the block-wide round trips through shared
+// and tensor memory bound the tcgen05 form (variant 8, bf16 activations): 14.5
+// GLUPS at 128^3.  Here a layer's accumulators are the next layer's operand in
+// the same registers, and nothing but the warp waits.
+// On CUDA cores the network took 1,344 fused multiply-adds a node: 11.3 GLUPS at
+// 128^3, 15.9 with this form (error of the step against 64 bits 9.5e-7 both).
+// ---------------------------------------------------------------------------
+constexpr int CLO_ROW = 80;  // bytes of a node's row of features: 32 bf16 padded, so that
+                             // eight rows of a matrix load hit distinct banks
+
+// fp32 values as sums of three bf16 numbers, two values a word.
+__device__ __forceinline__ void clo_split(float a, float b, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
+  auto pack = [](float x, float y) {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
+    return *reinterpret_cast<const uint32_t*>(&h);
+  };
+  hi = pack(a, b);
+  a = __fsub_rn(a, __uint_as_float(hi << 16));
+  b = __fsub_rn(b, __uint_as_float(hi & 0xffff0000u));
+  mid = pack(a, b);
+  a = __fsub_rn(a, __uint_as_float(mid << 16));
+  b = __fsub_rn(b, __uint_as_float(mid & 0xffff0000u));
+  lo = pack(a, b);
+}
+
+__device__ __forceinline__ void clo_mma_sync(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+      "{%0, %1, %2, %3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+// r of the warp's 32 nodes, lane = node, from their raw inputs.  Every lane of
+// the warp calls it.
+__device__ __forceinline__ float closure_warp(const CloNet<2>& w, const float (&xr)[CLO_IN]) {
+  __shared__ __align__(16) uint8_t rows[4][32 * CLO_ROW];  // blocks of up to four warps
+  const int lane = threadIdx.x & 31, t = lane & 3;
+  const int warp = (int)(threadIdx.y * blockDim.x + threadIdx.x) >> 5;
+  const uint4* __restrict__ frag = w.frag;
+  {
+    // k = 10 s + j: part s (high, middle, low) of feature j, 30 and 31 zero
+    float x[CLO_IN + 1];
+#pragma unroll
+    for (int j = 0; j < CLO_IN; ++j) x[j] = __fmul_rn(__fsub_rn(xr[j], w.v[CLO_MEAN + j]), w.v[CLO_ISCALE + j]);
+    x[CLO_IN] = 0.0f;
+    uint32_t k[16];
+#pragma unroll
+    for (int q = 0; q < 5; ++q) clo_split(x[2 * q], x[2 * q + 1], k[q], k[5 + q], k[10 + q]);
+    k[15] = 0u;
+    uint4* row = reinterpret_cast<uint4*>(rows[warp] + lane * CLO_ROW);
+    __syncwarp();  // the last evaluation has read its rows
+#pragma unroll
+    for (int q = 0; q < 4; ++q) row[q] = make_uint4(k[4 * q], k[4 * q + 1], k[4 * q + 2], k[4 * q + 3]);
+    __syncwarp();
+  }
+  float z0[2], z1[2];  // rows lane / 4 and lane / 4 + 8 of the two halves of the warp
+#pragma unroll
+  for (int m = 0; m < 2; ++m) {
+    auto bias = [&](int at, float (&c)[4][4]) {  // columns 8 j + 2 t and + 1 of both rows
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const uint4 b = __ldg(frag + 256 + (at + q) * 4 + t);
+        c[2 * q][0] = c[2 * q][2] = __uint_as_float(b.x);
+        c[2 * q][1] = c[2 * q][3] = __uint_as_float(b.y);
+        c[2 * q + 1][0] = c[2 * q + 1][2] = __uint_as_float(b.z);
+        c[2 * q + 1][1] = c[2 * q + 1][3] = __uint_as_float(b.w);
+      }
+    };
+    float c1[4][4];
+    bias(0, c1);
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+      uint32_t a[4];
+      const uint32_t at = (uint32_t)__cvta_generic_to_shared(rows[warp]) +
+                          (uint32_t)((16 * m + (lane & 15)) * CLO_ROW + 32 * s + 16 * (lane >> 4));
+      asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+                   : "=r"(a[0]), "=r"(a[1]), "=r"(a[2]), "=r"(a[3]) : "r"(at) : "memory");
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const uint4 b = __ldg(frag + (2 * s + q) * 32 + lane);
+        clo_mma_sync(c1[2 * q], a, b.x, b.y);
+        clo_mma_sync(c1[2 * q + 1], a, b.z, b.w);
+      }
+    }
+    float c2[4][4];
+    bias(2, c2);
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+      uint32_t a[3][4];  // columns 16 s .. 16 s + 15 of relu(c1) as an operand, in three parts
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int r = 0; r < 2; ++r)
+          clo_split(fmaxf(c1[2 * s + h][2 * r], 0.0f), fmaxf(c1[2 * s + h][2 * r + 1], 0.0f), a[2][2 * h + r],
+                    a[1][2 * h + r], a[0][2 * h + r]);
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const uint4 b = __ldg(frag + 128 + (2 * s + q) * 32 + lane);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {  // small parts first
+          clo_mma_sync(c2[2 * q], a[k], b.x, b.y);
+          clo_mma_sync(c2[2 * q + 1], a[k], b.z, b.w);
+        }
+      }
+    }
+    float s0 = 0.0f, s1 = 0.0f;
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const uint4 w3 = __ldg(frag + 256 + (4 + q) * 4 + t);
+      const float ww[4] = {__uint_as_float(w3.x), __uint_as_float(w3.y), __uint_as_float(w3.z), __uint_as_float(w3.w)};
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          s0 = __fmaf_rn(ww[2 * h + e], fmaxf(c2[2 * q + h][e], 0.0f), s0);
+          s1 = __fmaf_rn(ww[2 * h + e], fmaxf(c2[2 * q + h][2 + e], 0.0f), s1);
+        }
+    }
+#pragma unroll
+    for (int o = 1; o < 4; o <<= 1) {
+      s0 = __fadd_rn(s0, __shfl_xor_sync(0xffffffffu, s0, o));
+      s1 = __fadd_rn(s1, __shfl_xor_sync(0xffffffffu, s1, o));
+    }
+    z0[m] = s0;
+    z1[m] = s1;
+  }
+  // back to lane = node: row r of half m lies in lanes 4 (r mod 8) ..
+  const int src = 4 * (lane & 7);
+  const float a = __shfl_sync(0xffffffffu, z0[0], src), b = __shfl_sync(0xffffffffu, z1[0], src);
+  const float c = __shfl_sync(0xffffffffu, z0[1], src), d = __shfl_sync(0xffffffffu, z1[1], src);
+  const float z = (lane & 16) ? ((lane & 8) ? d : c) : ((lane & 8) ? b : a);
+  return Ops1::softplus(__fadd_rn(z, w.v[CLO_B3]));
+}
+__device__ __forceinline__ float closure_step_r(const CloNet<2>& w, const float (&x)[CLO_IN]) {
+  return closure_warp(w, x);
+}
+__device__ __forceinline__ float2 closure_step_r(const CloNet<2>& w, const float2 (&x)[CLO_IN]) {
+  float a[CLO_IN];
+#pragma unroll
+  for (int j = 0; j < CLO_IN; ++j) a[j] = x[j].x;
+  const float ra = closure_warp(w, a);
+#pragma unroll
+  for (int j = 0; j < CLO_IN; ++j) a[j] = x[j].y;
+  return make_float2(ra, closure_warp(w, a));
 }
 
 // The tensor-core evaluation of CloNet<3> (see there); every thread of the

@@ -127,7 +127,8 @@ void free_all(Ctx* c) {
   for (auto& g : c->graph)
     if (g) cudaGraphExecDestroy(g);
   void* ptrs[] = {c->fbuf[0], c->fbuf[1], c->pop,      c->mask,     c->flags, c->links,
-                  c->rho,     c->u,       c->status,   c->partials, c->sums,  c->staging};
+                  c->rho,     c->u,       c->status,   c->partials, c->sums,  c->staging,
+                  c->clo_frag};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (c->own_stream) cudaStreamDestroy(c->own_stream);
@@ -343,12 +344,23 @@ int lbm_set_closure(lbm_ctx* c, const float* net) {
     for (int k = 0; k < LBM_CLOSURE_FLOATS; ++k)
       if (!std::isfinite(net[k])) return fail(c, LBM_ERR_INVALID_ARG, "closure network has a non-finite value");
   }
+  if (net && !c->clo_frag) {
+    uint32_t* p = nullptr;
+    if (int rc = dev_alloc(c, &p, lbm::CLO_FRAG_WORDS, "cudaMalloc(closure)")) return rc;
+    c->clo_frag = p;
+  }
   // Captured step graphs hold the old network by value: rebuild them.
   CK(cudaStreamSynchronize(c->stream), "set_closure sync");
   drop_graphs(c);
   c->closure = net != nullptr;
   for (int k = 0; k < LBM_CLOSURE_FLOATS; ++k) {
     c->clo[k] = !net ? 0.f : lbm::clo_is_weight(k) ? lbm::round_bf16(net[k]) : net[k];
+  }
+  if (net) {
+    uint32_t words[lbm::CLO_FRAG_WORDS];
+    lbm::clo_fragments(c->clo, words);
+    CK(cudaMemcpyAsync(c->clo_frag, words, sizeof(words), cudaMemcpyHostToDevice, c->stream), "upload closure");
+    CK(cudaStreamSynchronize(c->stream), "upload closure sync");
   }
   return c->initialized ? prepare_graphs(c) : LBM_OK;
 }
@@ -546,7 +558,10 @@ int lbm_sync(lbm_ctx* c) {
   CK(cudaStreamSynchronize(c->stream), "sync");
   if (st) {
     CK(cudaMemsetAsync(c->status, 0, sizeof(unsigned), c->stream), "reset status");
-    if (st & 4u) return fail(c, LBM_ERR_TIMEOUT, "a step kernel's wait for its row copies gave up");
+    if (st & 4u) {
+      c->initialized = false;  // rows of the step are missing: the state is not whole
+      return fail(c, LBM_ERR_TIMEOUT, "a step kernel's wait for its row copies gave up");
+    }
     if (st & 2u)
       return fail(c, LBM_ERR_TIMEOUT, "the closure's tensor-core MMA wait gave up (nodes fell back to Smagorinsky)");
     return fail(c, LBM_ERR_NONFINITE, "non-finite value or rho <= 0 at a fluid node");

@@ -27,6 +27,13 @@ constexpr int CLO_MEAN = CLO_NPARAM;
 constexpr int CLO_ISCALE = CLO_MEAN + CLO_IN;
 constexpr int CLO_FLOATS = CLO_ISCALE + CLO_IN;    // 1427
 
+// The network's layers as the step kernels' matrix products read them
+// (closure_warp in closure.cuh), in 32-bit words: per lane and k step the B
+// operands of W1 (k = 10 s + j: feature j, three times) and of W2, then b1, b2
+// and W3 by the columns that lane mod 4 holds.
+constexpr int CLO_FRAG_WORDS = 4 * (128 + 128 + 24);
+void clo_fragments(const float* net, uint32_t* words);
+
 constexpr bool clo_is_weight(int k) {
   return (k >= CLO_W1 && k < CLO_B1) || (k >= CLO_W2 && k < CLO_B2) || (k >= CLO_W3 && k < CLO_B3);
 }
@@ -173,6 +180,7 @@ struct Ctx {
   // value; weights already rounded to bf16
   bool closure = false;
   float clo[LBM_CLOSURE_FLOATS] = {};
+  void* clo_frag = nullptr;   // device: its layers as matrix fragments (clo_fragments)
   uint32_t clo_wait_polls = LBM_CLO_WAIT_LIMIT;  // polls per tensor-core MMA wait
   // nodes per thread of the physics step: 0 automatic, 1, 2 or 4
   int step_variant = 0;

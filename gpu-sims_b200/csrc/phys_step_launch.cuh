@@ -33,20 +33,17 @@ namespace {
 #ifndef LBM_STEP2_MINB16_SMAG
 #define LBM_STEP2_MINB16_SMAG 5
 #endif
-// Residency bounds of the learned-closure kernels (the MLP's hidden layer
-// stays in registers: two nodes' worth in the pair kernel).
+// Residency bounds of the learned-closure kernels.  With the network on mma.sync
+// (closure_warp) they are bound by instruction issue and its latency, 2,285
+// instructions for 64 nodes, 0.51 a cycle and scheduler at three blocks; 128^3,
+// GLUPS at 2 / 3 / 4 / 5 blocks per SM: pair kernel fp32 12.1 / 14.4 / 15.9 / 12.8
+// (640 bytes spilled), fp16 14.7 / 14.7 / 17.4 / 16.5; one-node kernel at 3 / 5 / 6:
+// fp32 12.3 / 13.9 / 13.5, fp16 13.6 / 14.2 / 14.6.
 #ifndef LBM_CLO_MINB
-#define LBM_CLO_MINB 3
+#define LBM_CLO_MINB 5
 #endif
-// The pair kernel with the CUDA-core MLP, 128^3: fp32 storage at three
-// blocks per SM (168 registers, 32-124 bytes spilled) 11.3 GLUPS against 10.5
-// at two (208-220 registers, no spills); the 2-byte formats 11.7 against 11.9,
-// so they keep two.
 #ifndef LBM_CLO2_MINB
-#define LBM_CLO2_MINB 2
-#endif
-#ifndef LBM_CLO2_MINB32
-#define LBM_CLO2_MINB32 3
+#define LBM_CLO2_MINB 4
 #endif
 
 // Rows per block of the pair kernel.  One-warp blocks whose row is
@@ -69,7 +66,7 @@ constexpr int step2_rows() {
 // SGS: 0 none, 1 Smagorinsky, 2 learned closure (net = the network).
 template <int PREC, int COLL, int SGS, bool FORCE, bool WRITE_MOMENTS, int P>
 __global__ void __launch_bounds__(32 * step2_rows<PREC, SGS>(),
-                                  SGS == 2 ? (PREC == LBM_PREC_F32 ? LBM_CLO2_MINB32 : LBM_CLO2_MINB)
+                                  SGS == 2 ? LBM_CLO2_MINB
                                   : PREC == LBM_PREC_F32
                                       ? (SGS == 1 ? LBM_STEP2_MINB_SMAG : LBM_STEP2_MINB) * STEP_BY
                                       : (SGS == 1 ? LBM_STEP2_MINB16_SMAG : LBM_STEP2_MINB16) * STEP_BY /
@@ -275,6 +272,7 @@ template <int SGS> CloNet<SGS> net_of(const Ctx&) { return CloNet<SGS>{}; }
 template <> CloNet<2> net_of<2>(const Ctx& c) {
   CloNet<2> n;
   for (int k = 0; k < CLO_FLOATS; ++k) n.v[k] = c.clo[k];
+  n.frag = static_cast<const uint4*>(c.clo_frag);
   return n;
 }
 
@@ -415,11 +413,11 @@ cudaError_t launch_step_tc(const Ctx& c, int P, bool wm, cudaStream_t s) {
 }
 
 // CLOSURE: the learned-closure kernels (compiled in their own files; no body
-// force, which lbm_set_closure enforces): the CUDA-core MLP (one or two
-// nodes per thread, fp32 activations) by default, the tensor-core MLP (bf16
-// hidden activations) for variant 8.  Measured on B200 at 128^3: CUDA-core
-// pair kernel 11.3 / 11.9 GLUPS (fp32 / fp16 storage), tensor-core kernel
-// 14.5 / 15.8.
+// force, which lbm_set_closure enforces): the warp-level matrix products
+// (closure_warp, one or two nodes per thread, activations to fp32 accuracy) by
+// default, the tcgen05 MLP (bf16 activations) for variant 8.  Measured on B200 at
+// 128^3 (fp32 / fp16 storage): 15.9 / 17.4 GLUPS (11.3 / 12.0 with the network on
+// CUDA cores), tcgen05 14.4 / 15.8.
 template <int PREC, int COLL, bool CLOSURE>
 cudaError_t dispatch_smag(const Ctx& c, int P, bool wm, cudaStream_t s) {
   if constexpr (CLOSURE) {
