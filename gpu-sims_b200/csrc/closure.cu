@@ -171,31 +171,30 @@ __global__ void __launch_bounds__(256) k_predict(const float* __restrict__ net,
 // ---------------------------------------------------------------------------
 // Fused forward/backward of one batch.
 //
-// A warp takes 32 samples at a time, lane = sample, for the forward pass
-// and the backward pass through the activations; it leaves the per-sample
-// activations (h1, h2), pre-activation gradients (d a1, d a2), standardised
-// inputs and d z in shared memory.  The weight gradients are then
-// accumulated with lane = hidden unit: lane i owns row i of dW2 and dW1 and
-// entry i of db1, db2, dW3, so each sums its 32 samples with no atomics.
-// At the end the block's warps are summed in a fixed order into the
-// block's slot of `part` (one row of LBM_CLOSURE_PARAMS per block), which
-// the Adam kernel sums over blocks, again in a fixed order: the gradient is
-// deterministic.
+// A block takes 32 samples at a time, lane = sample, and its four warps share
+// them: warp w owns hidden units 8w .. 8w+7 of both layers, forward and backward,
+// and hands the activations (h1, h2) and pre-activation gradients (d a1, d a2) on
+// through shared memory.  The weight gradients are accumulated with lane =
+// hidden unit (row i of dW2 and dW1), warp w taking columns 8w .. 8w+7 of dW2 and
+// its share of the rest, each summing the 32 samples with no atomics.  At the
+// end the block's gradient goes to its row of `part`, which the Adam kernel sums
+// over blocks in a fixed order: the gradient is deterministic.
+// Bound by the latency of its sums at the batch sizes of training, by shared
+// loads beyond: a warp that took 32 samples by itself needed 3,900 steps for them
+// one after the other (batch of 4,096: 16.6 us on 32 SMs, and 6.2 us to sum over
+// blocks).  lbm_trainer_grad, gradient read back: 4,096 samples 48.5 -> 32.8 us,
+// 65,536 77 -> 62, 300,000 139 -> 139.
 // Sample j of the batch is dataset row (a * (start + j) + c) mod n.
 // ---------------------------------------------------------------------------
 constexpr int TR_WARPS = 4;
 constexpr int TR_THREADS = 32 * TR_WARPS;
-constexpr int TR_LD = 36;   // row stride of the per-warp [32][36] tiles: float4
-                            // stores of 8 lanes hit 32 distinct banks
+constexpr int TR_OWN = CLO_HID / TR_WARPS;  // hidden units of a warp
+constexpr int TR_LD = 36;   // row stride of the [32][36] tiles: float4 accesses of
+                            // 8 lanes hit 32 distinct banks
 constexpr int TR_XLD = 12;  // row stride of the inputs tile
-constexpr int TR_WARP_FLOATS = 4 * 32 * TR_LD + 32 * TR_XLD + 32;
-constexpr int TR_MAX_BLOCKS = 296;
-// the network copy is padded to a multiple of 4 floats so that every tile
-// after it starts on a 16-byte boundary (float4 accesses)
-constexpr int TR_NET = (CLO_FLOATS + 3) / 4 * 4;
-constexpr size_t TR_SMEM = (size_t)(TR_NET + CLO_HID * CLO_HID + TR_WARPS * TR_WARP_FLOATS) * 4;
-static_assert(TR_NET % 4 == 0 && (CLO_HID * CLO_HID) % 4 == 0 && TR_WARP_FLOATS % 4 == 0 &&
-                  TR_LD % 4 == 0 && TR_XLD % 4 == 0 && CLO_W2 % 4 == 0,
+constexpr int TR_MAX_BLOCKS = 592;  // four per SM
+constexpr int TR_NET = (CLO_FLOATS + 3) / 4 * 4;  // 16-byte multiple: float4 tiles follow
+static_assert(TR_LD % 4 == 0 && TR_XLD % 4 == 0 && CLO_W2 % 4 == 0 && CLO_HID * CLO_HID % 4 == 0 && TR_OWN == 8,
               "16-byte alignment of the float4 tiles");
 
 struct Batch {
@@ -209,43 +208,45 @@ struct Batch {
   float wscale;    // loss = wscale * sum w (r - t)^2
 };
 
-__global__ void __launch_bounds__(TR_THREADS, 2)
+__global__ void __launch_bounds__(TR_THREADS, 4)
     k_mlp_grad(const float* __restrict__ net, Batch B, float* __restrict__ part,
                double* __restrict__ loss_part) {
-  extern __shared__ __align__(16) float sm[];
-  float* sw = sm;                                       // network [CLO_FLOATS] (padded)
-  float* sW2T = sm + TR_NET;                            // W2 transposed [j][i]
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  float* wb = sW2T + CLO_HID * CLO_HID + warp * TR_WARP_FLOATS;
-  float* sH1 = wb;                  // [32][TR_LD] h1 per sample
-  float* sH2 = sH1 + 32 * TR_LD;    // h2
-  float* sA1 = sH2 + 32 * TR_LD;    // d a1
-  float* sA2 = sA1 + 32 * TR_LD;    // d a2
-  float* sX = sA2 + 32 * TR_LD;     // [32][TR_XLD] standardised inputs
-  float* sDZ = sX + 32 * TR_XLD;    // [32] d z
+  __shared__ __align__(16) float sw[TR_NET];                // the network
+  __shared__ __align__(16) float sW2T[CLO_HID * CLO_HID];   // W2 transposed [j][i]
+  __shared__ __align__(16) float sW1[CLO_HID * TR_XLD];     // W1 in rows of 12, the last three zero
+  __shared__ __align__(16) float sH1[32 * TR_LD], sH2[32 * TR_LD], sA1[32 * TR_LD], sA2[32 * TR_LD];
+  __shared__ __align__(16) float sX[32 * TR_XLD];           // standardised inputs
+  __shared__ float sDZ[32], sZ[TR_WARPS][32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, own = warp * TR_OWN;
 
   for (int k = threadIdx.x; k < CLO_FLOATS; k += TR_THREADS) sw[k] = net[k];
   for (int k = threadIdx.x; k < CLO_HID * CLO_HID; k += TR_THREADS) {
     const int i = k / CLO_HID, j = k % CLO_HID;
     sW2T[j * CLO_HID + i] = net[CLO_W2 + k];
   }
+  for (int k = threadIdx.x; k < CLO_HID * TR_XLD; k += TR_THREADS) {
+    const int i = k / TR_XLD, j = k % TR_XLD;
+    sW1[k] = j < CLO_IN ? net[CLO_W1 + i * CLO_IN + j] : 0.f;
+  }
   __syncthreads();
 
-  float gW2[CLO_HID], gW1[CLO_IN];
+  // lane = hidden unit i: dW2[i][own ..]; warp 0 dW1[i][0 .. 3], warp 1
+  // dW1[i][4 .. 7], warp 2 dW1[i][8] and db1[i], warp 3 db2[i], dW3[i] and db3
+  float gW2[TR_OWN], gr[4];
 #pragma unroll
-  for (int j = 0; j < CLO_HID; ++j) gW2[j] = 0.f;
+  for (int q = 0; q < TR_OWN; ++q) gW2[q] = 0.f;
 #pragma unroll
-  for (int k = 0; k < CLO_IN; ++k) gW1[k] = 0.f;
-  float gb1 = 0.f, gb2 = 0.f, gW3 = 0.f, gb3 = 0.f;
+  for (int q = 0; q < 4; ++q) gr[q] = 0.f;
   double lsum = 0.0;
 
   const int64_t groups = (B.nb + 31) / 32;
-  for (int64_t gi = (int64_t)blockIdx.x * TR_WARPS + warp; gi < groups;
-       gi += (int64_t)gridDim.x * TR_WARPS) {
-    // ---- forward and activation backward, lane = sample ----
+  for (int64_t gi = blockIdx.x; gi < groups; gi += gridDim.x) {
+    // ---- forward, lane = sample ----
     const int64_t j = gi * 32 + lane;
     const bool valid = j < B.nb;
-    float xs[CLO_IN];
+    float xs[TR_XLD];
+#pragma unroll
+    for (int k = 0; k < TR_XLD; ++k) xs[k] = 0.f;
     float tgt = 0.f, wt = 0.f;
     if (valid) {
       const uint64_t pos = (uint64_t)(B.start + j);
@@ -255,132 +256,139 @@ __global__ void __launch_bounds__(TR_THREADS, 2)
         xs[k] = (B.x[row * CLO_IN + k] - sw[CLO_MEAN + k]) * sw[CLO_ISCALE + k];
       tgt = B.t[row];
       wt = B.w[row];
-    } else {
-#pragma unroll
-      for (int k = 0; k < CLO_IN; ++k) xs[k] = 0.f;
     }
-    float h1[CLO_HID];
+    float v[TR_OWN];
 #pragma unroll
-    for (int i = 0; i < CLO_HID; ++i) {
-      float a = sw[CLO_B1 + i];
-#pragma unroll
-      for (int k = 0; k < CLO_IN; ++k) a = fmaf(sw[CLO_W1 + i * CLO_IN + k], xs[k], a);
-      h1[i] = fmaxf(a, 0.f);
+    for (int q = 0; q < TR_OWN; ++q) {
+      const float4* wr = reinterpret_cast<const float4*>(sW1 + (own + q) * TR_XLD);
+      const float4 w0 = wr[0], w1 = wr[1];
+      float a = sw[CLO_B1 + own + q];
+      a = fmaf(w0.w, xs[3], fmaf(w0.z, xs[2], fmaf(w0.y, xs[1], fmaf(w0.x, xs[0], a))));
+      a = fmaf(w1.w, xs[7], fmaf(w1.z, xs[6], fmaf(w1.y, xs[5], fmaf(w1.x, xs[4], a))));
+      a = fmaf(sW1[(own + q) * TR_XLD + 8], xs[8], a);
+      v[q] = fmaxf(a, 0.f);
     }
-    float z = sw[CLO_B3];
-    unsigned m2 = 0;
+    auto put8 = [&](float* tile) {  // the warp's eight units of this lane's sample
+      *reinterpret_cast<float4*>(tile + lane * TR_LD + own) = make_float4(v[0], v[1], v[2], v[3]);
+      *reinterpret_cast<float4*>(tile + lane * TR_LD + own + 4) = make_float4(v[4], v[5], v[6], v[7]);
+    };
+    put8(sH1);
+    if (warp == 0) {
 #pragma unroll
-    for (int i = 0; i < CLO_HID; i += 4) {
-      float h2v[4];
+      for (int k = 0; k < TR_XLD; k += 4)
+        *reinterpret_cast<float4*>(sX + lane * TR_XLD + k) = make_float4(xs[k], xs[k + 1], xs[k + 2], xs[k + 3]);
+    }
+    __syncthreads();
+    float z = 0.f;
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const float4* wr = reinterpret_cast<const float4*>(sw + CLO_W2 + (i + q) * CLO_HID);
-        float a = sw[CLO_B2 + i + q];
+    for (int q = 0; q < TR_OWN; ++q) v[q] = sw[CLO_B2 + own + q];
 #pragma unroll
-        for (int jj = 0; jj < CLO_HID / 4; ++jj) {
-          const float4 w4 = wr[jj];
-          a = fmaf(w4.x, h1[4 * jj], a);
-          a = fmaf(w4.y, h1[4 * jj + 1], a);
-          a = fmaf(w4.z, h1[4 * jj + 2], a);
-          a = fmaf(w4.w, h1[4 * jj + 3], a);
-        }
-        h2v[q] = fmaxf(a, 0.f);
-        if (a > 0.f) m2 |= 1u << (i + q);
-        z = fmaf(sw[CLO_W3 + i + q], h2v[q], z);
+    for (int j4 = 0; j4 < CLO_HID / 4; ++j4) {
+      const float4 h = *reinterpret_cast<const float4*>(sH1 + lane * TR_LD + 4 * j4);
+#pragma unroll
+      for (int q = 0; q < TR_OWN; ++q) {
+        const float4 w4 = *reinterpret_cast<const float4*>(sw + CLO_W2 + (own + q) * CLO_HID + 4 * j4);
+        v[q] = fmaf(w4.w, h.w, fmaf(w4.z, h.z, fmaf(w4.y, h.y, fmaf(w4.x, h.x, v[q]))));
       }
-      *reinterpret_cast<float4*>(sH2 + lane * TR_LD + i) = make_float4(h2v[0], h2v[1], h2v[2], h2v[3]);
     }
 #pragma unroll
-    for (int i = 0; i < CLO_HID; i += 4)
-      *reinterpret_cast<float4*>(sH1 + lane * TR_LD + i) = make_float4(h1[i], h1[i + 1], h1[i + 2], h1[i + 3]);
-    // softplus output and the weighted squared error
+    for (int q = 0; q < TR_OWN; ++q) {
+      v[q] = fmaxf(v[q], 0.f);
+      z = fmaf(sw[CLO_W3 + own + q], v[q], z);
+    }
+    put8(sH2);
+    sZ[warp][lane] = z;
+    __syncthreads();
+    // softplus output and the weighted squared error (in every warp: the same)
+    z = sw[CLO_B3] + ((sZ[0][lane] + sZ[1][lane]) + (sZ[2][lane] + sZ[3][lane]));
     const float r = z > 20.f ? z : log1pf(expf(z));
     const float sig = 1.f / (1.f + expf(-z));
     const float e = r - tgt;
     const float dz = valid ? 2.f * B.wscale * wt * e * sig : 0.f;
-    if (valid) lsum += (double)B.wscale * (double)wt * (double)e * (double)e;
-    float da2[CLO_HID];
+    if (valid && warp == 0) lsum += (double)B.wscale * (double)wt * (double)e * (double)e;
+    if (warp == 0) sDZ[lane] = dz;
 #pragma unroll
-    for (int i = 0; i < CLO_HID; ++i) da2[i] = (m2 >> i & 1u) ? sw[CLO_W3 + i] * dz : 0.f;
-#pragma unroll
-    for (int i = 0; i < CLO_HID; i += 4)
-      *reinterpret_cast<float4*>(sA2 + lane * TR_LD + i) = make_float4(da2[i], da2[i + 1], da2[i + 2], da2[i + 3]);
+    for (int q = 0; q < TR_OWN; ++q) v[q] = v[q] > 0.f ? sw[CLO_W3 + own + q] * dz : 0.f;
+    put8(sA2);
+    __syncthreads();
     // d a1_j = [a1_j > 0] sum_i W2[i][j] d a2_i  (W2 transposed: row j contiguous)
 #pragma unroll
-    for (int jq = 0; jq < CLO_HID; jq += 4) {
-      float d[4];
+    for (int q = 0; q < TR_OWN; ++q) v[q] = 0.f;
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int jj = jq + q;
-        const float4* wr = reinterpret_cast<const float4*>(sW2T + jj * CLO_HID);
-        float a = 0.f;
+    for (int i4 = 0; i4 < CLO_HID / 4; ++i4) {
+      const float4 d = *reinterpret_cast<const float4*>(sA2 + lane * TR_LD + 4 * i4);
 #pragma unroll
-        for (int i4 = 0; i4 < CLO_HID / 4; ++i4) {
-          const float4 w4 = wr[i4];
-          a = fmaf(w4.x, da2[4 * i4], a);
-          a = fmaf(w4.y, da2[4 * i4 + 1], a);
-          a = fmaf(w4.z, da2[4 * i4 + 2], a);
-          a = fmaf(w4.w, da2[4 * i4 + 3], a);
-        }
-        d[q] = h1[jj] > 0.f ? a : 0.f;
+      for (int q = 0; q < TR_OWN; ++q) {
+        const float4 w4 = *reinterpret_cast<const float4*>(sW2T + (own + q) * CLO_HID + 4 * i4);
+        v[q] = fmaf(w4.w, d.w, fmaf(w4.z, d.z, fmaf(w4.y, d.y, fmaf(w4.x, d.x, v[q]))));
       }
-      *reinterpret_cast<float4*>(sA1 + lane * TR_LD + jq) = make_float4(d[0], d[1], d[2], d[3]);
     }
+    {
+      const float4 h0 = *reinterpret_cast<const float4*>(sH1 + lane * TR_LD + own);
+      const float4 h1 = *reinterpret_cast<const float4*>(sH1 + lane * TR_LD + own + 4);
+      const float h[TR_OWN] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
 #pragma unroll
-    for (int k = 0; k < CLO_IN; ++k) sX[lane * TR_XLD + k] = xs[k];
-    sDZ[lane] = dz;
-    __syncwarp();
+      for (int q = 0; q < TR_OWN; ++q) v[q] = h[q] > 0.f ? v[q] : 0.f;
+    }
+    put8(sA1);
+    __syncthreads();
     // ---- weight gradients, lane = hidden unit ----
-    for (int s = 0; s < 32; ++s) {
+    auto sample = [&](int s) {  // dW2 of one sample; its d a2
       const float a2 = sA2[s * TR_LD + lane];
-      const float a1 = sA1[s * TR_LD + lane];
-      const float dzs = sDZ[s];
-      const float4* h = reinterpret_cast<const float4*>(sH1 + s * TR_LD);
+      const float4 h0 = *reinterpret_cast<const float4*>(sH1 + s * TR_LD + own);
+      const float4 h1 = *reinterpret_cast<const float4*>(sH1 + s * TR_LD + own + 4);
+      const float h[TR_OWN] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
 #pragma unroll
-      for (int q = 0; q < CLO_HID / 4; ++q) {
-        const float4 hv = h[q];
-        gW2[4 * q] = fmaf(a2, hv.x, gW2[4 * q]);
-        gW2[4 * q + 1] = fmaf(a2, hv.y, gW2[4 * q + 1]);
-        gW2[4 * q + 2] = fmaf(a2, hv.z, gW2[4 * q + 2]);
-        gW2[4 * q + 3] = fmaf(a2, hv.w, gW2[4 * q + 3]);
+      for (int q = 0; q < TR_OWN; ++q) gW2[q] = fmaf(a2, h[q], gW2[q]);
+      return a2;
+    };
+    if (warp < 2) {
+#pragma unroll 4
+      for (int s = 0; s < 32; ++s) {
+        sample(s);
+        const float a1 = sA1[s * TR_LD + lane];
+        const float4 x = *reinterpret_cast<const float4*>(sX + s * TR_XLD + 4 * warp);
+        gr[0] = fmaf(a1, x.x, gr[0]);
+        gr[1] = fmaf(a1, x.y, gr[1]);
+        gr[2] = fmaf(a1, x.z, gr[2]);
+        gr[3] = fmaf(a1, x.w, gr[3]);
       }
-#pragma unroll
-      for (int k = 0; k < CLO_IN; ++k) gW1[k] = fmaf(a1, sX[s * TR_XLD + k], gW1[k]);
-      gb1 += a1;
-      gb2 += a2;
-      gW3 = fmaf(dzs, sH2[s * TR_LD + lane], gW3);
-      gb3 += dzs;
+    } else if (warp == 2) {
+#pragma unroll 4
+      for (int s = 0; s < 32; ++s) {
+        sample(s);
+        const float a1 = sA1[s * TR_LD + lane];
+        gr[0] = fmaf(a1, sX[s * TR_XLD + 8], gr[0]);
+        gr[1] += a1;
+      }
+    } else {
+#pragma unroll 4
+      for (int s = 0; s < 32; ++s) {
+        gr[0] += sample(s);
+        gr[1] = fmaf(sDZ[s], sH2[s * TR_LD + lane], gr[1]);
+        gr[2] += sDZ[s];
+      }
     }
-    __syncwarp();
+    __syncthreads();  // the tiles are rewritten by the next samples
   }
 
-  // ---- block reduction in a fixed order ----
-  // loss: warp sum (butterfly, the same order on every run), then warps in order
-  for (int o = 16; o > 0; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
-  __syncthreads();  // every warp is done with its tiles
-  float* g = wb;    // this warp's gradient row, CLO_NPARAM floats (fits the tiles)
+  float* row = part + (size_t)blockIdx.x * CLO_NPARAM;
 #pragma unroll
-  for (int jj = 0; jj < CLO_HID; ++jj) g[CLO_W2 + lane * CLO_HID + jj] = gW2[jj];
+  for (int q = 0; q < TR_OWN; ++q) row[CLO_W2 + lane * CLO_HID + own + q] = gW2[q];
+  if (warp < 2) {
 #pragma unroll
-  for (int k = 0; k < CLO_IN; ++k) g[CLO_W1 + lane * CLO_IN + k] = gW1[k];
-  g[CLO_B1 + lane] = gb1;
-  g[CLO_B2 + lane] = gb2;
-  g[CLO_W3 + lane] = gW3;
-  if (lane == 0) g[CLO_B3] = gb3;
-  __shared__ double sl[TR_WARPS];
-  if (lane == 0) sl[warp] = lsum;
-  __syncthreads();
-  const float* g0 = sW2T + CLO_HID * CLO_HID;
-  for (int k = threadIdx.x; k < CLO_NPARAM; k += TR_THREADS) {
-    float acc = g0[k];
-#pragma unroll
-    for (int w = 1; w < TR_WARPS; ++w) acc += g0[w * TR_WARP_FLOATS + k];
-    part[(size_t)blockIdx.x * CLO_NPARAM + k] = acc;
+    for (int q = 0; q < 4; ++q) row[CLO_W1 + lane * CLO_IN + 4 * warp + q] = gr[q];
+  } else if (warp == 2) {
+    row[CLO_W1 + lane * CLO_IN + 8] = gr[0];
+    row[CLO_B1 + lane] = gr[1];
+  } else {
+    row[CLO_B2 + lane] = gr[0];
+    row[CLO_W3 + lane] = gr[1];
+    if (lane == 0) row[CLO_B3] = gr[2];
   }
-  if (threadIdx.x == 0) {
-    double l = 0.0;
-    for (int w = 0; w < TR_WARPS; ++w) l += sl[w];
-    loss_part[blockIdx.x] = l;
+  if (warp == 0) {  // butterfly: the same order on every run
+    for (int o = 16; o > 0; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
+    if (lane == 0) loss_part[blockIdx.x] = lsum;
   }
 }
 
@@ -388,24 +396,40 @@ struct AdamArgs {
   float lr, b1, b2, eps, wd;
   float bc1, bc2;   // 1 - beta^t
   int apply;        // 0: only reduce the gradient
+  int set_loss;     // 1: the loss is set, 0: added to loss_acc
 };
 
-// Sums the block partials (fixed order), then optionally one Adam step of
-// the fp32 master parameters; writes the network the kernels use (weights
-// rounded to bf16).  Thread 0 adds the batch loss to loss_acc.
-__global__ void k_adam(const float* __restrict__ part, int nblk, const double* __restrict__ loss_part,
-                       double* __restrict__ loss_acc, float* __restrict__ grad,
-                       float* __restrict__ theta, float* __restrict__ m, float* __restrict__ v,
-                       float* __restrict__ net, AdamArgs A) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k == 0) {
+// Sums the block partials, then optionally one Adam step of the fp32 master
+// parameters; writes the network the kernels use (weights rounded to bf16).  A
+// block takes 32 parameters, its eight warps every eighth block's partial, and
+// adds the warps' sums in order: the same result on every run, in an eighth of
+// the loads one after the other.  The first block adds the batch loss to
+// loss_acc (or sets it).
+constexpr int ADAM_THREADS = 256;
+__global__ void __launch_bounds__(ADAM_THREADS)
+    k_adam(const float* __restrict__ part, int nblk, const double* __restrict__ loss_part,
+           double* __restrict__ loss_acc, float* __restrict__ grad,
+           float* __restrict__ theta, float* __restrict__ m, float* __restrict__ v,
+           float* __restrict__ net, AdamArgs A) {
+  __shared__ float sums[ADAM_THREADS / 32][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int k = blockIdx.x * 32 + lane;
+  if (blockIdx.x == 0 && warp == 1) {
     double l = 0.0;
-    for (int b = 0; b < nblk; ++b) l += loss_part[b];
-    *loss_acc += l;
+    for (int b = lane; b < nblk; b += 32) l += loss_part[b];
+    for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
+    if (lane == 0) *loss_acc = A.set_loss ? l : *loss_acc + l;
   }
-  if (k >= CLO_NPARAM) return;
   float gk = 0.f;
-  for (int b = 0; b < nblk; ++b) gk += part[(size_t)b * CLO_NPARAM + k];
+  if (k < CLO_NPARAM) {
+#pragma unroll 8
+    for (int b = warp; b < nblk; b += ADAM_THREADS / 32) gk += part[(size_t)b * CLO_NPARAM + k];
+  }
+  sums[warp][lane] = gk;
+  __syncthreads();
+  if (warp != 0 || k >= CLO_NPARAM) return;
+#pragma unroll
+  for (int w = 1; w < ADAM_THREADS / 32; ++w) gk += sums[w][lane];
   grad[k] = gk;
   if (!A.apply) return;
   const float mk = A.b1 * m[k] + (1.f - A.b1) * gk;
@@ -448,12 +472,13 @@ struct lbm_trainer {
   float* theta = nullptr;   // fp32 master parameters [CLO_NPARAM]
   float* m = nullptr;
   float* v = nullptr;
-  float* grad = nullptr;    // last reduced gradient
+  float* grad = nullptr;    // last reduced gradient (behind loss_acc, in its allocation)
   float* net = nullptr;     // network the kernels use [CLO_FLOATS]
   float* part = nullptr;    // [TR_MAX_BLOCKS][CLO_NPARAM]
   double* loss_part = nullptr;
   double* loss_acc = nullptr;
   double* wpart = nullptr;  // [TR_MAX_BLOCKS]
+  char* host = nullptr;     // pinned: loss, gradient
   int64_t t = 0;            // Adam steps taken
   std::string err = "no error";
 };
@@ -482,30 +507,20 @@ int tcuda(lbm_trainer* t, cudaError_t e, const char* what) {
     if (e_ != cudaSuccess) return tcuda(t, e_, what);   \
   } while (0)
 
-bool grad_kernel_ready(cudaError_t* e) {
-  static cudaError_t once = cudaFuncSetAttribute(k_mlp_grad, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 (int)TR_SMEM);
-  *e = once;
-  return once == cudaSuccess;
-}
-
 int grid_for(int64_t nb) {
-  const int64_t groups = (nb + 31) / 32;
-  const int64_t blocks = (groups + TR_WARPS - 1) / TR_WARPS;
+  const int64_t blocks = (nb + 31) / 32;
   return (int)(blocks < 1 ? 1 : blocks > TR_MAX_BLOCKS ? TR_MAX_BLOCKS : blocks);
 }
 
 int launch_grad(lbm_trainer* t, const Batch& B, int* nblk) {
-  cudaError_t e;
-  if (!grad_kernel_ready(&e)) return tcuda(t, e, "closure grad kernel attribute");
   const int g = grid_for(B.nb);
-  k_mlp_grad<<<g, TR_THREADS, TR_SMEM, t->stream>>>(t->net, B, t->part, t->loss_part);
+  k_mlp_grad<<<g, TR_THREADS, 0, t->stream>>>(t->net, B, t->part, t->loss_part);
   TCK(t, cudaGetLastError(), "closure grad kernel");
   *nblk = g;
   return LBM_OK;
 }
 
-int launch_adam(lbm_trainer* t, int nblk, bool apply) {
+int launch_adam(lbm_trainer* t, int nblk, bool apply, bool set_loss) {
   AdamArgs A{};
   A.lr = t->opt.lr;
   A.b1 = t->opt.beta1;
@@ -513,6 +528,7 @@ int launch_adam(lbm_trainer* t, int nblk, bool apply) {
   A.eps = t->opt.eps;
   A.wd = t->opt.weight_decay;
   A.apply = apply ? 1 : 0;
+  A.set_loss = set_loss ? 1 : 0;
   if (apply) {
     t->t += 1;
     A.bc1 = (float)(1.0 - std::pow((double)A.b1, (double)t->t));
@@ -520,7 +536,7 @@ int launch_adam(lbm_trainer* t, int nblk, bool apply) {
   } else {
     A.bc1 = A.bc2 = 1.f;
   }
-  k_adam<<<(CLO_NPARAM + 255) / 256, 256, 0, t->stream>>>(t->part, nblk, t->loss_part, t->loss_acc,
+  k_adam<<<(CLO_NPARAM + 31) / 32, ADAM_THREADS, 0, t->stream>>>(t->part, nblk, t->loss_part, t->loss_acc,
                                                           t->grad, t->theta, t->m, t->v, t->net, A);
   TCK(t, cudaGetLastError(), "closure adam kernel");
   return LBM_OK;
@@ -619,11 +635,11 @@ int lbm_trainer_create(const float* net, const lbm_adam* opt, lbm_trainer** out)
   t->opt = o;
   struct A { void** p; size_t bytes; } allocs[] = {
       {reinterpret_cast<void**>(&t->theta), CLO_NPARAM * 4}, {reinterpret_cast<void**>(&t->m), CLO_NPARAM * 4},
-      {reinterpret_cast<void**>(&t->v), CLO_NPARAM * 4},     {reinterpret_cast<void**>(&t->grad), CLO_NPARAM * 4},
+      {reinterpret_cast<void**>(&t->v), CLO_NPARAM * 4},
       {reinterpret_cast<void**>(&t->net), CLO_FLOATS * 4},
       {reinterpret_cast<void**>(&t->part), (size_t)TR_MAX_BLOCKS * CLO_NPARAM * 4},
       {reinterpret_cast<void**>(&t->loss_part), TR_MAX_BLOCKS * 8},
-      {reinterpret_cast<void**>(&t->loss_acc), 8}, {reinterpret_cast<void**>(&t->wpart), TR_MAX_BLOCKS * 8}};
+      {reinterpret_cast<void**>(&t->loss_acc), 8 + CLO_NPARAM * 4}, {reinterpret_cast<void**>(&t->wpart), TR_MAX_BLOCKS * 8}};
   for (auto& a : allocs) {
     cudaError_t e = cudaMalloc(a.p, a.bytes);
     if (e != cudaSuccess) {
@@ -631,6 +647,12 @@ int lbm_trainer_create(const float* net, const lbm_adam* opt, lbm_trainer** out)
       lbm_trainer_destroy(t);
       return rc;
     }
+  }
+  t->grad = reinterpret_cast<float*>(t->loss_acc + 1);
+  if (cudaError_t e = cudaMallocHost(reinterpret_cast<void**>(&t->host), 8 + CLO_NPARAM * 4)) {
+    const int rc = tcuda(nullptr, e, "trainer: cudaMallocHost");
+    lbm_trainer_destroy(t);
+    return rc;
   }
   std::vector<float> h(CLO_FLOATS);
   for (int k = 0; k < CLO_FLOATS; ++k) h[k] = clo_is_weight(k) ? round_bf16(net[k]) : net[k];
@@ -650,9 +672,10 @@ int lbm_trainer_create(const float* net, const lbm_adam* opt, lbm_trainer** out)
 
 int lbm_trainer_destroy(lbm_trainer* t) {
   if (!t) return LBM_OK;
-  void* ptrs[] = {t->theta, t->m, t->v, t->grad, t->net, t->part, t->loss_part, t->loss_acc, t->wpart};
+  void* ptrs[] = {t->theta, t->m, t->v, t->net, t->part, t->loss_part, t->loss_acc, t->wpart};
   for (void* p : ptrs)
     if (p) cudaFree(p);
+  if (t->host) cudaFreeHost(t->host);
   delete t;
   return LBM_OK;
 }
@@ -670,14 +693,13 @@ int lbm_trainer_grad(lbm_trainer* t, const float* d_x, const float* d_target, co
   if (!d_x || !d_target || !d_weight || n <= 0) return tfail(t, LBM_ERR_INVALID_ARG, "trainer grad: bad batch");
   Batch B{d_x, d_target, d_weight, n, 0, n, 1, 0, wscale};
   int nblk = 0;
-  TCK(t, cudaMemsetAsync(t->loss_acc, 0, 8, t->stream), "trainer grad: reset loss");
   if (int rc = launch_grad(t, B, &nblk)) return rc;
-  if (int rc = launch_adam(t, nblk, false)) return rc;
-  if (grad) TCK(t, cudaMemcpyAsync(grad, t->grad, CLO_NPARAM * 4, cudaMemcpyDeviceToHost, t->stream), "trainer grad: read");
-  double l = 0.0;
-  TCK(t, cudaMemcpyAsync(&l, t->loss_acc, 8, cudaMemcpyDeviceToHost, t->stream), "trainer grad: read loss");
+  if (int rc = launch_adam(t, nblk, false, true)) return rc;
+  // gradient and loss in one copy to pinned memory
+  TCK(t, cudaMemcpyAsync(t->host, t->loss_acc, 8 + CLO_NPARAM * 4, cudaMemcpyDeviceToHost, t->stream), "trainer grad: read");
   TCK(t, cudaStreamSynchronize(t->stream), "trainer grad: sync");
-  if (loss) *loss = l;
+  if (grad) std::memcpy(grad, t->host + 8, CLO_NPARAM * 4);
+  if (loss) std::memcpy(loss, t->host, 8);
   return LBM_OK;
 }
 
@@ -687,7 +709,7 @@ int lbm_trainer_adam_step(lbm_trainer* t) {
   // partial row that the Adam kernel sums
   TCK(t, cudaMemcpyAsync(t->part, t->grad, CLO_NPARAM * 4, cudaMemcpyDeviceToDevice, t->stream), "trainer adam: stage");
   TCK(t, cudaMemsetAsync(t->loss_part, 0, 8, t->stream), "trainer adam: loss");
-  if (int rc = launch_adam(t, 1, true)) return rc;
+  if (int rc = launch_adam(t, 1, true, false)) return rc;
   return LBM_OK;
 }
 
@@ -731,7 +753,7 @@ int lbm_trainer_fit(lbm_trainer* t, const float* d_x, const float* d_target, con
       Batch B{d_x, d_target, d_weight, n, s, nb, a, c, (float)(1.0 / (wmean * (double)nb))};
       int nblk = 0;
       if (int rc = launch_grad(t, B, &nblk)) return rc;
-      if (int rc = launch_adam(t, nblk, true)) return rc;
+      if (int rc = launch_adam(t, nblk, true, false)) return rc;
       ++nbatches;
     }
     if (epoch_loss) {
