@@ -40,6 +40,13 @@ struct lbm_batch {
   cudaStream_t own = nullptr, stream = nullptr;
   cudaGraphExec_t graph[2] = {nullptr, nullptr};
   static constexpr int kGraphSteps = 16;
+  // graph mode's lanes (plan_lanes): each a list of domains, run one after the
+  // other, the lanes side by side on lane_blocks blocks each; empty: one tile
+  // launch a step
+  std::vector<std::vector<int>> lanes;
+  int lane_blocks = 0;
+  std::vector<cudaStream_t> lane_streams;  // for the capture
+  std::vector<cudaEvent_t> lane_events;
   int parity = 0;
   uint64_t total_nodes = 0, iteration = 0, dev_bytes = 0;
   void* staging = nullptr;
@@ -185,15 +192,100 @@ bool valid_schedule(const lbm_batch_schedule& s) {
          s.test_missing_blocks >= 0;
 }
 
+// Lanes of graph mode.  Domains do not touch each other, so within a graph each
+// may take its kGraphSteps steps by itself: a lane advances its domains one
+// after the other with the single-domain row-tile step (phys_rows.cuh) on its
+// share of the chip's 296 blocks, and the lanes run side by side.  A lane's
+// domain stays in L2 for its sixteen steps, which one launch over all domains
+// cannot give.  Domains go to lanes longest first; the number of lanes is the
+// one with the shortest estimate, and the tile kernel keeps batches where that
+// is no shorter than its own.  Estimates from B200: a round of tiles (one per
+// block) 2.2 us in 2-byte storage and 3.7 us in fp32, 4 us to start and end a
+// launch; the tile kernel 35.7 and 26.5 nodes/ns.
+void plan_lanes(lbm_batch* b) {
+  b->lanes.clear();
+  const size_t nd = b->dom.size();
+  const bool f32 = b->precision == LBM_PREC_F32;
+  const double round_us = f32 ? 3.7 : 2.2, launch_us = 4.0;
+  std::vector<uint32_t> tiles(nd);
+  for (size_t i = 0; i < nd; ++i)
+    if (!(tiles[i] = lbm::phys_rows_tiles(b->dom[i].pp.g))) return;
+  std::vector<int> order(nd);
+  for (size_t i = 0; i < nd; ++i) order[i] = (int)i;
+  std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return tiles[x] > tiles[y]; });
+  double best = 0.95 * (double)b->total_nodes / (f32 ? 26.5e3 : 35.7e3);  // us a step
+  for (int n : {2, 4, 8, 16}) {
+    if ((size_t)n > nd) break;
+    const int blocks = 296 / n;
+    std::vector<double> load(n, 0.0);
+    std::vector<std::vector<int>> lanes(n);
+    for (int d : order) {
+      const size_t l = std::min_element(load.begin(), load.end()) - load.begin();
+      load[l] += launch_us + round_us * ((tiles[d] + blocks - 1) / blocks);
+      lanes[l].push_back(d);
+    }
+    const double t = *std::max_element(load.begin(), load.end());
+    if (t < best) {
+      best = t;
+      b->lanes = std::move(lanes);
+      b->lane_blocks = blocks;
+    }
+  }
+}
+
+// Captures the lanes' steps from parity `slot` on b->own and its side streams.
+cudaError_t capture_lanes(lbm_batch* b, int slot) {
+  cudaError_t e = cudaSuccess;
+  auto ok = [&](cudaError_t r) {
+    if (e == cudaSuccess) e = r;
+    return e == cudaSuccess;
+  };
+  for (size_t l = 0; l < b->lanes.size(); ++l) {
+    cudaStream_t s = l ? b->lane_streams[l - 1] : b->own;
+    if (l == 0) ok(cudaEventRecord(b->lane_events[0], b->own));
+    else ok(cudaStreamWaitEvent(s, b->lane_events[0], 0));
+  }
+  for (size_t l = 0; l < b->lanes.size() && e == cudaSuccess; ++l) {
+    cudaStream_t s = l ? b->lane_streams[l - 1] : b->own;
+    for (int d : b->lanes[l]) {
+      b->dom[d].row_blocks = b->lane_blocks;
+      int P = slot;
+      for (int i = 0; i < lbm_batch::kGraphSteps && e == cudaSuccess; ++i, P ^= 1)
+        ok(b->precision == LBM_PREC_F32    ? lbm::phys_rows_f32(b->dom[d], P, false, s)
+           : b->precision == LBM_PREC_F16S ? lbm::phys_rows_f16(b->dom[d], P, false, s)
+                                           : lbm::phys_rows_bf16(b->dom[d], P, false, s));
+    }
+    if (l) ok(cudaEventRecord(b->lane_events[l], s));
+  }
+  for (size_t l = 1; l < b->lanes.size(); ++l) {
+    const cudaError_t r = cudaStreamWaitEvent(b->own, b->lane_events[l], 0);
+    if (e == cudaSuccess) e = r;
+  }
+  return e;
+}
+
 // Captures kGraphSteps steps from parity `slot`, without the moment write:
-// kGraphSteps launches of the tile kernel, or in persistent mode one
+// the lanes' steps, kGraphSteps launches of the tile kernel, or in persistent mode one
 // cooperative launch that takes all of them with grid barriers between.
 int build_graph(lbm_batch* b, int slot) {
   const lbm::BatchLaunch L = launch_of(b);
   cudaGraph_t g = nullptr;
+  const bool lanes = !b->sched.persistent && !b->lanes.empty();
+  while (lanes && b->lane_streams.size() + 1 < b->lanes.size()) {
+    cudaStream_t s = nullptr;
+    BCK(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking), "lane stream");
+    b->lane_streams.push_back(s);
+  }
+  while (lanes && b->lane_events.size() < b->lanes.size()) {
+    cudaEvent_t v = nullptr;
+    BCK(cudaEventCreateWithFlags(&v, cudaEventDisableTiming), "lane event");
+    b->lane_events.push_back(v);
+  }
   BCK(cudaStreamBeginCapture(b->own, cudaStreamCaptureModeThreadLocal), "begin capture");
   cudaError_t e = cudaSuccess;
-  if (b->sched.persistent) {
+  if (lanes) {
+    e = capture_lanes(b, slot);
+  } else if (b->sched.persistent) {
     e = lbm::batch_persistent(L, lbm_batch::kGraphSteps, slot, b->grid, b->own, false);
   } else {
     int P = slot;
@@ -380,6 +472,7 @@ int lbm_batch_create(const lbm_desc* descs, int n, lbm_batch** out) {
     const int per[3] = {v.d.periodic[0], v.d.periodic[1], v.d.periodic[2]};
     if (cudaError_t e = lbm::classify(v, per, b->stream)) return bail(bcuda(b, e, "classify"));
   }
+  plan_lanes(b);
   if (int rc = build_tiles(b)) return bail(rc);
   *out = b;
   return LBM_OK;
@@ -389,6 +482,8 @@ int lbm_batch_destroy(lbm_batch* b) {
   if (!b) return LBM_OK;
   if (b->stream) cudaStreamSynchronize(b->stream);
   drop_graphs(b);
+  for (auto s : b->lane_streams) cudaStreamDestroy(s);
+  for (auto v : b->lane_events) cudaEventDestroy(v);
   for (void* p : b->allocs) cudaFree(p);
   if (b->own) cudaStreamDestroy(b->own);
   delete b;
@@ -474,10 +569,11 @@ int lbm_batch_sync(lbm_batch* b) {
   if (st) {
     BCK(cudaMemsetAsync(b->status, 0, sizeof(unsigned), b->stream), "reset status");
     BCK(cudaStreamSynchronize(b->stream), "sync");
-    if (st & lbm::BATCH_STATUS_TIMEOUT) {
-      // The persistent kernel stopped between steps; the state is not a
-      // whole number of steps any more.
+    if (st & (lbm::BATCH_STATUS_TIMEOUT | lbm::BATCH_STATUS_ROWS)) {
+      // The kernel stopped between steps (persistent mode) or within one; the
+      // state is not a whole number of steps any more.
       for (size_t i = 0; i < b->ready.size(); ++i) b->ready[i] = false;
+      if (st & lbm::BATCH_STATUS_ROWS) return bfail(b, LBM_ERR_TIMEOUT, "a step kernel's wait for its row copies gave up");
       return bfail(b, LBM_ERR_TIMEOUT, "a grid-barrier wait of the persistent step gave up");
     }
     return bfail(b, LBM_ERR_NONFINITE, "non-finite value or rho <= 0 at a fluid node");

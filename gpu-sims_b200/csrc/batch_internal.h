@@ -17,6 +17,7 @@ namespace lbm {
 
 constexpr unsigned BATCH_STATUS_NONFINITE = 1u;  // same bit the single-domain step sets
 constexpr unsigned BATCH_STATUS_TIMEOUT = 2u;    // a grid-barrier wait gave up
+constexpr unsigned BATCH_STATUS_ROWS = 4u;       // a row tile's wait gave up (phys_rows.cuh)
 
 // One domain as the batched kernels see it (copied to shared memory per tile).
 struct BatchDomain {

@@ -123,6 +123,8 @@ cudaError_t phys_step_bf16(const Ctx& c, int parity, bool write_moments, cudaStr
 cudaError_t phys_rows_f32(const Ctx& c, int parity, bool write_moments, cudaStream_t s);
 cudaError_t phys_rows_f16(const Ctx& c, int parity, bool write_moments, cudaStream_t s);
 cudaError_t phys_rows_bf16(const Ctx& c, int parity, bool write_moments, cudaStream_t s);
+// the number of its tiles for a grid, 0 where rows do not fit
+uint32_t phys_rows_tiles(const PhysGeom& g);
 cudaError_t phys_step_clo_f32(const Ctx& c, int parity, bool write_moments, cudaStream_t s);
 cudaError_t phys_step_clo_f16(const Ctx& c, int parity, bool write_moments, cudaStream_t s);
 cudaError_t phys_step_clo_bf16(const Ctx& c, int parity, bool write_moments, cudaStream_t s);
@@ -182,6 +184,9 @@ struct Ctx {
   float clo[LBM_CLOSURE_FLOATS] = {};
   void* clo_frag = nullptr;   // device: its layers as matrix fragments (clo_fragments)
   uint32_t clo_wait_polls = LBM_CLO_WAIT_LIMIT;  // polls per tensor-core MMA wait
+  // blocks of a row-tile step, 0: the whole chip's (a batch runs several domains
+  // side by side)
+  int row_blocks = 0;
   // nodes per thread of the physics step: 0 automatic, 1, 2 or 4
   int step_variant = 0;
   bool initialized = false;

@@ -749,7 +749,7 @@ cudaError_t launch_row_tiles(const Ctx& c, int P, cudaStream_t s) {
   auto* fn = &k_phys_rows<PREC, COLL, SGS, FORCE, WM, OPEN>;
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  const uint32_t most = 148u * (deep ? 1 : rows_blocks<PREC, SGS>());
+  const uint32_t most = c.row_blocks ? (uint32_t)c.row_blocks : 148u * (deep ? 1 : rows_blocks<PREC, SGS>());
   const dim3 grd(rt.ntiles < most ? rt.ntiles : most);
   fn<<<grd, ROWS_THREADS, smem, s>>>(c.pp, rt, c.pop, c.flags, c.links, c.rho, c.u, c.status, P);
   return cudaGetLastError();
