@@ -400,7 +400,7 @@ def run_ours(args, world, rank, local):
                      "peak_kind": ("measured copy bandwidth (MEASURED_PEAKS.json hbm_gbs)" if peak_kind == "measured"
                                    else "fallback copy bandwidth (6650 GB/s, an earlier measurement on this pool; "
                                         "MEASURED_PEAKS.json absent)"),
-                     "kernel": "k_phys_step2 (fused esoteric-pull stream+collide, two nodes per thread)"},
+                     "kernel": "k_phys_rows (fused esoteric-pull stream+collide, rows streamed through shared memory)"},
         "variants": runs,
         "e2e": e2e,
         "gpu_launches": args.steps,

@@ -253,7 +253,7 @@ __global__ void __launch_bounds__(256) k_predict(const float* __restrict__ net,
 // Bound by the latency of its sums at the batch sizes of training, by shared
 // loads beyond: a warp that took 32 samples by itself needed 3,900 steps for them
 // one after the other (batch of 4,096: 16.6 us on 32 SMs, and 6.2 us to sum over
-// blocks).  lbm_trainer_grad, gradient read back: 4,096 samples 48.5 -> 32.8 us,
+// blocks).  lbm_trainer_grad, gradient read back: 4,096 samples 46.8 -> 33.6 us,
 // 65,536 77 -> 62, 300,000 139 -> 139.
 // Sample j of the batch is dataset row (a * (start + j) + c) mod n.
 // ---------------------------------------------------------------------------

@@ -19,8 +19,9 @@
 
 namespace lbm {
 
-// Network handed to a step kernel by value: in the kernel's parameter space
-// every weight is a constant-bank operand of its FMA.  Kernels without the
+// Network handed to a step kernel by value: biases, input scaling and the
+// weights of kernels that run a layer on CUDA cores are constant-bank operands;
+// the matrix products read their fragments from `frag`.  Kernels without the
 // closure take the one-float placeholder.
 template <int SGS> struct CloNet {
   float v[1];

@@ -199,8 +199,8 @@ def run_duct(steps=1000, shape=(512, 128, 128)):
 def run_closure_step(n=128, steps=200, variants=(0, 1, 8)):
     """The learned-closure step on an n^3 periodic box (tau 0.502, Cs0 0.1, a
     He-initialised network, seeded random velocity): MLUPS per step variant
-    (0 automatic: CUDA-core MLP, two nodes per thread; 1 one node per
-    thread; 8 tensor-core MLP) in fp32 and fp16 storage."""
+    (0 automatic: warp-level matrix products, two nodes per thread; 1 the
+    same, one node per thread; 8 tcgen05 MLP) in fp32 and fp16 storage."""
     from lbm import closure as cl
     stream, timed = _timer()
     net = cl.init_net(5, np.zeros(lbm.CLOSURE_INPUTS), np.ones(lbm.CLOSURE_INPUTS))

@@ -229,7 +229,8 @@ LBM_API int lbm_set_params(lbm_ctx* ctx, const lbm_params* params);
 /* Waits for the context's stream; returns LBM_ERR_NONFINITE if a NaN/Inf or
  * non-positive density was seen at a fluid node since the last sync, and
  * LBM_ERR_TIMEOUT if a learned-closure step's bounded wait for its
- * tensor-core MMA gave up (those nodes used plain Smagorinsky). */
+ * tensor-core MMA gave up (those nodes used plain Smagorinsky) or a step's
+ * bounded wait for its row copies did (the state then needs a new init). */
 LBM_API int lbm_sync(lbm_ctx* ctx);
 
 /* Copies rho (float[N]) and u (format u_fmt) to host memory; either pointer
@@ -448,8 +449,10 @@ LBM_API int lbm_jitter_lut(uint8_t* out);
 
 /* ---- batched ensemble --------------------------------------------------- */
 /* Hundreds of independent physics-mode domains of uneven size advanced
- * together: one launch per step over a tile work-list (captured in a CUDA
- * graph), or one persistent cooperative launch per lbm_batch_step call.  The
+ * together: in a CUDA graph, as parallel lanes that take each domain sixteen
+ * steps at a time or as one launch per step over a tile work-list, whichever
+ * is estimated shorter; or one persistent cooperative launch per
+ * lbm_batch_step call.  The
  * reference runs one domain at a time (src/main.cpp:1554-1591); a batch is
  * equivalent to lbm_step on each domain alone, bit for bit. */
 typedef struct lbm_batch lbm_batch;
@@ -488,7 +491,8 @@ LBM_API int lbm_batch_init_from_moments(lbm_batch* b, int domain, const float* r
                                         const void* u, int u_fmt);
 LBM_API int lbm_batch_step(lbm_batch* b, int nsteps);
 /* LBM_ERR_NONFINITE as lbm_sync; LBM_ERR_TIMEOUT if a persistent launch's
- * grid barrier gave up (the domains then need a new init). */
+ * grid barrier or a step's wait for its row copies gave up (the domains then
+ * need a new init). */
 LBM_API int lbm_batch_sync(lbm_batch* b);
 LBM_API int lbm_batch_read_moments(lbm_batch* b, int domain, float* rho, void* u, int u_fmt);
 LBM_API int lbm_batch_read_populations(lbm_batch* b, int domain, float* f, size_t n);
