@@ -747,7 +747,11 @@ cudaError_t launch_row_tiles(const Ctx& c, int P, cudaStream_t s) {
   if (PREC == LBM_PREC_F32 && !deep) rt.stages = 2;
   const size_t smem = (size_t)rt.stages * rows_stage<PREC>();
   auto* fn = &k_phys_rows<PREC, COLL, SGS, FORCE, WM, OPEN>;
-  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  // The limit belongs to the kernel, which all lattices of the process share (other
+  // threads' and captured graphs' among them): always that of the most stages,
+  // never lowered to this launch's.
+  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       ROWS_MAXST * rows_stage<PREC>());
   if (e != cudaSuccess) return e;
   const uint32_t most = c.row_blocks ? (uint32_t)c.row_blocks : 148u * (deep ? 1 : rows_blocks<PREC, SGS>());
   const dim3 grd(rt.ntiles < most ? rt.ntiles : most);
