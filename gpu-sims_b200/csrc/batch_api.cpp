@@ -710,6 +710,11 @@ int lbm_batch_get_info(lbm_batch* b, lbm_batch_info* info) {
   return LBM_OK;
 }
 
+int lbm_batch_lanes(lbm_batch* b) {
+  if (!b) return bfail(nullptr, LBM_ERR_INVALID_ARG, "batch is NULL");
+  return b->sched.persistent ? 0 : (int)b->lanes.size();
+}
+
 const char* lbm_batch_last_error(lbm_batch* b) { return b ? b->err.c_str() : lbm_last_error(nullptr); }
 
 }  // extern "C"

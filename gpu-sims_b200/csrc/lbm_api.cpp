@@ -333,6 +333,12 @@ int lbm_set_step_variant(lbm_ctx* c, int nodes_per_thread) {
   return c->initialized ? prepare_graphs(c) : LBM_OK;
 }
 
+int lbm_step_streams_rows(lbm_ctx* c) {
+  if (int rc = check_ctx(c)) return rc;
+  return c->d.mode == LBM_MODE_PHYSICS && c->step_variant == 0 && !c->closure &&
+         lbm::phys_rows_pay(c->pp.g, c->d.precision);
+}
+
 int lbm_set_closure(lbm_ctx* c, const float* net) {
   if (int rc = check_ctx(c)) return rc;
   if (c->d.mode != LBM_MODE_PHYSICS) return fail(c, LBM_ERR_UNSUPPORTED, "the closure needs physics mode");

@@ -284,31 +284,8 @@ inline bool use_quads(const Ctx& c) {
   if (c.closure || c.pp.any_open || nx % 4) return false;
   return c.step_variant == 4 || (c.step_variant == 0 && step_quads(nx));
 }
-// Row tiles (phys_rows.cuh) by default where rows fill their blocks and the
-// grid has enough tiles to fill the persistent blocks (148 or 296) several
-// times; else the row kernels' small blocks win.  The lines, measured on B200
-// (row tiles / row kernels, GLUPS):
-//  * rows below 66 nodes waste padding and tiles: 64^3 22.8 / 30.2 (fp16), 56 x
-//    56 x 200 29.5 / 36.2 (fp32), 57 x 57 x 200 26.0 / 31.0 (fp16);
-//  * nodes per 512-node tile: fp32 144^3 (0.84) 36.6 / 31.9, 200 x 97 x 120 (0.78)
-//    34.7 / 32.4, 385 x 97 x 120 (0.75) 32.9 / 31.4, 180 x 97 x 120 (0.70) 32.2 / 33.8,
-//    257 x 97 x 120 (0.50) 24.7 / 30.2; fp16 200 x 97 x 120 53.3 / 43.0, 192^3 (0.75)
-//    48.8 / 58.4, 320 x 97 x 120 (0.63) 54.9 / 56.5; odd rows, which only the one-node
-//    kernel takes otherwise, pay in 2-byte storage at any fill (257 43.3 / 35.1);
-//  * rows that leave the row kernels' 64-wide warps ragged: fp16 72^3 (792 tiles)
-//    27.2 / 23.4, fp32 72^3 24.2 / 24.2, 80^3 (1,120) 29.7 / 28.4;
-//  * rows of whole warps: fp16 128^3 (4,096) 56.1 / 55.6, 256 x 256 x 8 (1,024)
-//    45.1 / 51.9; fp32 256 x 128 x 128 (8,192) 37.8 / 38.3, 512 x 128 x 128 (16,384)
-//    41.2 / 39.4, 256^3 (32,768) 42.5 / 41.6.
 inline bool use_row_tiles(const Ctx& c) {
-  if (c.step_variant != 0 || c.closure) return false;
-  const int nx = c.pp.g.nx;
-  const RowTiles rt = row_tiles(c.pp.g);
-  if (rt.R == 0 || nx < 66) return false;
-  const bool odd = nx % 2 != 0, whole = !odd && 20 * ((nx + 63) / 64 * 64) <= 23 * nx;
-  const int fill = 100 * rt.R * nx / 512;  // per cent of a tile
-  if (c.d.precision == LBM_PREC_F32) return fill >= 74 && rt.ntiles >= (whole ? 12000u : 1000u);
-  return (odd || fill >= 76) && rt.ntiles >= (whole ? 4000u : 700u);
+  return c.step_variant == 0 && !c.closure && row_tiles_pay(c.pp.g, c.d.precision);
 }
 inline bool use_pairs(const Ctx& c) {
   const int nx = c.pp.g.nx;

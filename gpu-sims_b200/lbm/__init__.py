@@ -221,6 +221,8 @@ _SIGS = {
     "lbm_render_velmag": (C.c_int, [_P, _I32, _I32, _I32, C.POINTER(VelmagParams), _I32, _I32, _P, _P]),
     "lbm_colormap_lut": (C.c_int, [_P]),
     "lbm_jitter_lut": (C.c_int, [_P]),
+    "lbm_step_streams_rows": (C.c_int, [_P]),
+    "lbm_batch_lanes": (C.c_int, [_P]),
     "lbm_set_closure": (C.c_int, [_P, _P]),
     "lbm_set_closure_wait_limit": (C.c_int, [_P, C.c_int32]),
     "lbm_box_filter": (C.c_int, [_P, _P, _I32, _I32, _I32, _I32, _P, _P]),
@@ -437,6 +439,10 @@ class Lattice:
         """F9: restores a capture (see lbm_capture_load)."""
         self._c(load().lbm_capture_load(self._h, str(capture_dir).encode(), flags))
 
+    def streams_rows(self) -> bool:
+        """Whether step() streams rows through shared memory (lbm_step_streams_rows)."""
+        return load().lbm_step_streams_rows(self._h) == 1
+
     def set_closure(self, net: np.ndarray | None) -> None:
         """Installs a learned-closure network (float[CLOSURE_FLOATS]); None
         removes it."""
@@ -598,6 +604,10 @@ class Batch:
         s.struct_size = C.sizeof(BatchSchedule)
         self._c(load().lbm_batch_autotune(self._h, trial_steps, C.byref(s)))
         return s
+
+    def lanes(self) -> int:
+        """Parallel lanes that graph mode runs (lbm_batch_lanes)."""
+        return load().lbm_batch_lanes(self._h)
 
     def info(self) -> BatchInfo:
         i = BatchInfo()

@@ -206,6 +206,11 @@ LBM_API int lbm_step(lbm_ctx* ctx, int nsteps);
  * knob; LBM_ERR_UNSUPPORTED for a variant the grid or precision cannot use. */
 LBM_API int lbm_set_step_variant(lbm_ctx* ctx, int nodes_per_thread);
 
+/* 1 when lbm_step streams rows through shared memory (the automatic choice for
+ * this grid, precision, variant and closure), 0 when it runs another kernel;
+ * < 0 on error. */
+LBM_API int lbm_step_streams_rows(lbm_ctx* ctx);
+
 /* The parameters in effect (from the descriptor, or the last lbm_set_params). */
 LBM_API int lbm_get_params(lbm_ctx* ctx, lbm_params* params);
 
@@ -503,6 +508,10 @@ LBM_API int lbm_batch_get_schedule(lbm_batch* b, lbm_batch_schedule* s);
  * are cached per (precision, collision, size class) for the process and, if
  * $LBM_AUTOTUNE_CACHE names a file, across processes. */
 LBM_API int lbm_batch_autotune(lbm_batch* b, int trial_steps, lbm_batch_schedule* best);
+/* The parallel lanes that graph mode runs (16 steps of whole domains side by
+ * side), 0 when it launches the tile kernel or the batch is in persistent mode;
+ * < 0 on error. */
+LBM_API int lbm_batch_lanes(lbm_batch* b);
 LBM_API int lbm_batch_get_info(lbm_batch* b, lbm_batch_info* info);
 LBM_API const char* lbm_batch_last_error(lbm_batch* b);
 

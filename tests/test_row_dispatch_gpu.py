@@ -1,0 +1,86 @@
+"""Which kernel the automatic choice and graph mode take, so that the tests that
+compare row tiles with another kernel do compare two kernels; and the forms of
+the row tiles that those tests do not reach."""
+import numpy as np
+import pytest
+
+from test_batch_lanes_gpu import initial
+from test_row_tiles import CASES, test_matches_one_node_kernel as matches_one_node_kernel
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("prec", [0, 1, 2])
+def test_choice_by_grid_variant_and_closure(gpu, prec):
+    for c in CASES.values():
+        nx, ny, nz = c["shape"]
+        lat = gpu.Lattice(nx=nx, ny=ny, nz=nz, mode=gpu.MODE_PHYSICS, precision=prec,
+                          periodic=c.get("periodic", (0, 0, 0)), tau=0.57, smagorinsky_cs=c.get("cs", 0.0))
+        assert lat.streams_rows(), c
+        lat.set_step_variant(1)
+        assert not lat.streams_rows()
+        lat.close()
+    lat = gpu.Lattice(nx=64, ny=64, nz=64, mode=gpu.MODE_PHYSICS, precision=prec, tau=0.6)
+    assert not lat.streams_rows()
+    lat.close()
+
+
+@pytest.mark.parametrize("case", [dict(shape=(160, 100, 100), lid=True, sphere=True),
+                                  dict(shape=(161, 101, 101), periodic=(1, 0, 1), sphere=True, trt=True)])
+def test_five_stage_fp32(gpu, monkeypatch, case):
+    """fp32 above 120 MB without Smagorinsky: one block an SM, five stages."""
+    monkeypatch.setitem(CASES, "deep", case)
+    lat = gpu.Lattice(nx=case["shape"][0], ny=case["shape"][1], nz=case["shape"][2], mode=gpu.MODE_PHYSICS,
+                      periodic=case.get("periodic", (0, 0, 0)), tau=0.57)
+    assert lat.streams_rows()
+    lat.close()
+    matches_one_node_kernel(gpu, 0, "deep")
+
+
+LANES = {  # shape, periodic: batches that graph mode runs in lanes
+    "fp32": (0, [((64, 64, 64), (0, 0, 0)), ((101, 60, 50), (0, 0, 0)), ((96, 66, 60), (0, 1, 0)),
+                 ((66, 64, 64), (1, 1, 1)), ((127, 40, 60), (0, 0, 1)), ((64, 48, 80), (0, 0, 0)),
+                 ((128, 56, 50), (1, 0, 1))] * 2),
+    # with a domain of the five-stage form beside two-stage ones
+    "fp32_deep": (0, [((160, 100, 100), (0, 0, 0)), ((64, 64, 64), (0, 0, 0)), ((128, 56, 50), (1, 0, 1)),
+                      ((96, 66, 60), (0, 1, 0)), ((66, 64, 64), (1, 1, 1)), ((127, 40, 60), (0, 0, 1)),
+                      ((64, 48, 80), (0, 0, 0)), ((101, 60, 50), (0, 0, 0))]),
+    "fp16": (1, [((96, 80, 40), (0, 0, 0)), ((71, 50, 40), (1, 0, 1)), ((33, 60, 70), (0, 0, 0)),
+                 ((80, 80, 80), (0, 0, 1))] * 4),
+}
+
+
+@pytest.mark.parametrize("name", sorted(LANES))
+def test_lanes_run_and_equal_single_domains(gpu, name):
+    """Every domain bit for bit as advanced alone by the one-node kernel, over
+    graphs from both parities and the launches after them."""
+    prec, specs = LANES[name]
+    wall = np.zeros((6, 3))
+    wall[gpu.FACE_ZP] = (0.04, 0, 0)
+    descs = [gpu.default_desc(nx=s[0], ny=s[1], nz=s[2], mode=gpu.MODE_PHYSICS, precision=prec,
+                              periodic=per, tau=0.55 + 0.02 * i, wall_velocity=wall)
+             for i, (s, per) in enumerate(specs)]
+    b = gpu.Batch(descs)
+    assert b.lanes() > 0
+    for i, d in enumerate(descs):
+        mask, rho, u = initial(d, i)
+        b.set_flags(i, mask)
+        b.init_from_moments(i, rho, u)
+    b.step(19)
+    b.step(35)
+    b.sync()
+    for i, d in enumerate(descs):
+        mask, rho, u = initial(d, i)
+        lat = gpu.Lattice(d)
+        lat.set_flags(mask)
+        lat.init_from_moments(rho, u)
+        lat.set_step_variant(1)
+        lat.step(54)
+        assert np.array_equal(b.read_populations(i), lat.read_populations()), i
+        assert all(np.array_equal(x, y) for x, y in zip(b.read_moments(i), lat.read_moments())), i
+        lat.close()
+    b.close()
+    b = gpu.Batch(descs)
+    b.set_schedule(persistent=1)
+    assert b.lanes() == 0
+    b.close()
