@@ -710,6 +710,14 @@ int lbm_batch_get_info(lbm_batch* b, lbm_batch_info* info) {
   return LBM_OK;
 }
 
+int lbm_batch_set_row_wait_limit(lbm_batch* b, int32_t polls) {
+  if (!b) return bfail(nullptr, LBM_ERR_INVALID_ARG, "batch is NULL");
+  BCK(cudaStreamSynchronize(b->stream), "set_row_wait_limit sync");
+  drop_graphs(b);
+  for (auto& v : b->dom) v.row_wait_polls = polls < 0 ? (uint32_t)LBM_ROW_WAIT_LIMIT : (uint32_t)polls;
+  return LBM_OK;
+}
+
 int lbm_batch_lanes(lbm_batch* b) {
   if (!b) return bfail(nullptr, LBM_ERR_INVALID_ARG, "batch is NULL");
   return b->sched.persistent ? 0 : (int)b->lanes.size();

@@ -73,6 +73,10 @@ struct PhysGeom {
 #ifndef LBM_CLO_WAIT_LIMIT
 #define LBM_CLO_WAIT_LIMIT (1 << 22)
 #endif
+// ... and of a row-tile step's waits for its copies (lbm_set_row_wait_limit)
+#ifndef LBM_ROW_WAIT_LIMIT
+#define LBM_ROW_WAIT_LIMIT (1 << 22)
+#endif
 
 struct PhysParams {
   PhysGeom g;
@@ -189,6 +193,7 @@ struct Ctx {
   // blocks of a row-tile step, 0: the whole chip's (a batch runs several domains
   // side by side)
   int row_blocks = 0;
+  uint32_t row_wait_polls = LBM_ROW_WAIT_LIMIT;  // polls of the collision's wait for a tile's rows
   // nodes per thread of the physics step: 0 automatic, 1, 2 or 4
   int step_variant = 0;
   bool initialized = false;

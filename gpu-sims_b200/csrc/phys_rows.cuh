@@ -46,7 +46,8 @@ constexpr int ROWS_CONS = 256;   // consumer threads
 constexpr int ROWS_SERV = 4;     // service warps, which issue the copies
 constexpr int ROWS_MAXST = 5;
 // polls of a wait (each try_wait suspends for a while) before the block gives up
-constexpr uint32_t ROWS_WAIT_LIMIT = 1u << 22;
+// (Ctx::row_wait_polls for the collision's wait for its rows)
+constexpr uint32_t ROWS_WAIT_LIMIT = LBM_ROW_WAIT_LIMIT;
 
 // One array's part of a stage: the tile's elements, then a 4-byte slot per
 // row for the x face's value.
@@ -101,10 +102,10 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
       : "=r"(done) : "r"(bar), "r"(parity) : "memory");
   return done != 0;
 }
-// Bounded wait: false when it ran out or another warp of the block gave up.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile uint32_t* abort) {
-  if (mbar_try(bar, parity)) return true;
-  for (uint32_t i = 0; i < ROWS_WAIT_LIMIT; ++i) {
+// Bounded wait: false when it ran out (at once with no polls) or another warp of
+// the block gave up.
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile uint32_t* abort, uint32_t polls) {
+  for (uint32_t i = 0; i < polls; ++i) {
     if (mbar_try(bar, parity)) return true;
     if (*abort) return false;
   }
@@ -255,6 +256,7 @@ __host__ __device__ __forceinline__ ptrdiff_t side_offset(const PhysGeom& G, int
 // The barriers of a block's stages, and its abort mark.
 struct RowBars {
   uint32_t full, done;  // shared addresses: rows landed, nodes collided
+  uint32_t* loaded;     // shared, per service warp: tiles it has loaded (rows_drain)
   volatile uint32_t* abort;
   unsigned* status;
   __device__ __forceinline__ void give_up() const {
@@ -278,6 +280,22 @@ struct RowStage {
 __device__ __forceinline__ bool inner_tile(const PhysGeom& G, int y0, int z, int rows) {
   return y0 > 0 && y0 + rows < G.ny && z > 0 && z < G.nz - 1;
 }
+// A block that gives up leaves no load in flight.  A tile's `full` phase takes
+// the arrivals of all service warps, and they may have stopped at different
+// tiles: a warp that loaded `mine` tiles, where the one furthest ahead loaded
+// `most`, first arrives for those it left out, and then every load of the block
+// shows in the phases of the last `stages` tiles.  Those waits end: a warp loads
+// tile t only when tile t - stages is collided, so all have loaded that one, the
+// tiles between mine and most lie in different stages, and their phases are the
+// stages' current ones.  arrive(stage) makes a warp's whole arrival, wait(stage,
+// parity) waits for a phase.
+template <class ARRIVE, class WAIT>
+__host__ __device__ __forceinline__ void rows_drain(uint32_t mine, uint32_t most, uint32_t stages, ARRIVE&& arrive,
+                                                    WAIT&& wait) {
+  for (uint32_t t = mine; t < most; ++t) arrive(t % stages);
+  for (uint32_t t = most > stages ? most - stages : 0; t < most; ++t) wait(t % stages, (t / stages) & 1u);
+}
+
 constexpr int ROWS_NA = (Q + ROWS_SERV - 1) / ROWS_SERV;  // arrays of a service warp: part, part + ROWS_SERV, ...
 constexpr uint64_t ROWS_MOST_BYTES = 1ull << 36;          // of a store (32-bit offsets of 16 bytes, below)
 
@@ -366,7 +384,7 @@ __device__ __forceinline__ bool rows_service(const PhysGeom& G, const RowSeg& sg
   bool ok = true;
 #pragma unroll 1
   for (uint32_t j = 0; j < sg.count; ++j) {
-    ok = __all_sync(FULL, mbar_wait(B.done + 8 * st_.s, st_.ph, B.abort));
+    ok = __all_sync(FULL, mbar_wait(B.done + 8 * st_.s, st_.ph, B.abort, ROWS_WAIT_LIMIT));
     if (!ok) {
       B.give_up();
       break;
@@ -407,15 +425,27 @@ __device__ __forceinline__ bool rows_service(const PhysGeom& G, const RowSeg& sg
   }
   if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
   __syncwarp();
-  if (!ok) {
-    // leave no load in flight: each stage's current phase, if it has loads
-    for (uint32_t k = 0; k < stages && k < loaded; ++k) {
-      for (uint32_t i = 0; i < ROWS_WAIT_LIMIT; ++i)
-        if (mbar_try(B.full + 8 * st_.s, st_.ph)) break;
-      st_.next(stages);
-    }
+  if (lane == 0) B.loaded[part] = loaded;
+  uint32_t any;  // of the service warps, gave up
+  asm volatile("{\n\t.reg .pred P1, P2;\n\tsetp.ne.u32 P1, %1, 0;\n\t"
+               "barrier.cta.red.or.pred P2, 1, %2, P1;\n\tselp.b32 %0, 1, 0, P2;\n\t}\n"
+               : "=r"(any) : "r"(ok ? 0u : 1u), "n"(32 * ROWS_SERV) : "memory");
+  if (any) {
+    const volatile uint32_t* n = B.loaded;
+    uint32_t most = 0;
+    for (int w = 0; w < ROWS_SERV; ++w) most = max(most, n[w]);
+    rows_drain(
+        loaded, most, stages,
+        [&](uint32_t s) {
+          if (lane == 0)
+            asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], 33;" ::"r"(B.full + 8 * s) : "memory");
+        },
+        [&](uint32_t s, uint32_t parity) {
+          for (uint32_t i = 0; i < ROWS_WAIT_LIMIT; ++i)
+            if (mbar_try(B.full + 8 * s, parity)) break;
+        });
   }
-  return ok;
+  return !any;
 }
 
 // One pair of nodes' step on a landed tile: stream from, and collide into, the
@@ -630,7 +660,7 @@ struct RowDomain {
 template <int PREC, int COLL, int SGS, bool FORCE, bool WRITE_MOMENTS, bool OPEN>
 __device__ __forceinline__ bool rows_consume(const PhysParams& p, const PhysParams& cp, const PhysGeom& G, int moving,
                                              const RowSeg& sg, const RowDomain& D, uint8_t* sm, int tid, int P,
-                                             const RowBars& B, uint32_t stages, RowStage& st_) {
+                                             const RowBars& B, uint32_t polls, uint32_t stages, RowStage& st_) {
   const RowPair q = row_pair<PREC>(G, sg.rt.R, sg.rt.tpr, tid);
   RowWalk w;
   w.start(sg.first, sg.stride, sg.rt.tiles_y);
@@ -645,7 +675,7 @@ __device__ __forceinline__ bool rows_consume(const PhysParams& p, const PhysPara
       z = w.z;
       fl = row_flags(G, D.flags, q, y, z);
     }
-    if (!__all_sync(FULL, mbar_wait(B.full + 8 * st_.s, st_.ph, B.abort))) {
+    if (!__all_sync(FULL, mbar_wait(B.full + 8 * st_.s, st_.ph, B.abort, polls))) {
       B.give_up();
       return false;
     }
@@ -664,13 +694,15 @@ __device__ __forceinline__ bool rows_consume(const PhysParams& p, const PhysPara
 // called as segs(f) and calls f(p, cp, G, moving, segment, domain) for the
 // block's segments in order until f returns false.
 template <int PREC, int COLL, int SGS, bool FORCE, bool WRITE_MOMENTS, bool OPEN, class SEGS>
-__device__ __forceinline__ void rows_block(uint32_t stages, uint32_t cons_warps, unsigned* status, int P, SEGS&& segs) {
+__device__ __forceinline__ void rows_block(uint32_t stages, uint32_t cons_warps, uint32_t polls, unsigned* status, int P,
+                                           SEGS&& segs) {
   extern __shared__ __align__(128) uint8_t sm[];
   __shared__ __align__(8) uint64_t bars[2 * ROWS_MAXST];
-  __shared__ uint32_t s_abort;
+  __shared__ uint32_t s_abort, s_loaded[ROWS_SERV];
   RowBars B;
   B.full = smem_addr(bars);
   B.done = B.full + 8 * ROWS_MAXST;
+  B.loaded = s_loaded;
   B.abort = &s_abort;
   B.status = status;
   if (threadIdx.x == 0) {
@@ -697,7 +729,7 @@ __device__ __forceinline__ void rows_block(uint32_t stages, uint32_t cons_warps,
   segs([&](const PhysParams& p, const PhysParams& cp, const PhysGeom& G, int moving, const RowSeg& sg,
            const RowDomain& D) {
     return rows_consume<PREC, COLL, SGS, FORCE, WRITE_MOMENTS, OPEN>(p, cp, G, moving, sg, D, sm,
-                                                                           (int)threadIdx.x - 32 * ROWS_SERV, P, B, stages, st);
+                                                                           (int)threadIdx.x - 32 * ROWS_SERV, P, B, polls, stages, st);
   });
 }
 
@@ -706,12 +738,13 @@ template <int PREC, int COLL, int SGS, bool FORCE, bool WRITE_MOMENTS, bool OPEN
 __global__ void __launch_bounds__(ROWS_THREADS, rows_blocks<PREC, SGS>())
     k_phys_rows(const __grid_constant__ PhysParams p, RowTiles rt, void* __restrict__ pop_v,
                 const uint8_t* __restrict__ flags, const uint32_t* __restrict__ links,
-                float* __restrict__ rho_o, float* __restrict__ u_o, unsigned* __restrict__ status, int P) {
+                float* __restrict__ rho_o, float* __restrict__ u_o, unsigned* __restrict__ status, int P,
+                uint32_t polls) {
   const RowDomain D{pop_v, flags, links, rho_o, u_o};
   const RowSeg sg{rt, blockIdx.x, gridDim.x,
                   rt.ntiles <= blockIdx.x ? 0u : (rt.ntiles - blockIdx.x + gridDim.x - 1) / gridDim.x};
   const uint32_t cons_warps = (uint32_t)(rt.R * rt.tpr + 31) / 32;  // warps that have nodes
-  rows_block<PREC, COLL, SGS, FORCE, WRITE_MOMENTS, OPEN>((uint32_t)rt.stages, cons_warps, status, P, [&](auto&& f) {
+  rows_block<PREC, COLL, SGS, FORCE, WRITE_MOMENTS, OPEN>((uint32_t)rt.stages, cons_warps, polls, status, P, [&](auto&& f) {
     if (sg.count) f(p, p, p.g, p.any_moving_wall, sg, D);
   });
 }
@@ -781,7 +814,7 @@ cudaError_t launch_row_tiles(const Ctx& c, int P, cudaStream_t s) {
   if (e != cudaSuccess) return e;
   const uint32_t most = c.row_blocks ? (uint32_t)c.row_blocks : 148u * (deep ? 1 : rows_blocks<PREC, SGS>());
   const dim3 grd(rt.ntiles < most ? rt.ntiles : most);
-  fn<<<grd, ROWS_THREADS, smem, s>>>(c.pp, rt, c.pop, c.flags, c.links, c.rho, c.u, c.status, P);
+  fn<<<grd, ROWS_THREADS, smem, s>>>(c.pp, rt, c.pop, c.flags, c.links, c.rho, c.u, c.status, P, c.row_wait_polls);
   return cudaGetLastError();
 }
 

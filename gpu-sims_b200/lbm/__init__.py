@@ -222,7 +222,9 @@ _SIGS = {
     "lbm_colormap_lut": (C.c_int, [_P]),
     "lbm_jitter_lut": (C.c_int, [_P]),
     "lbm_step_streams_rows": (C.c_int, [_P]),
+    "lbm_set_row_wait_limit": (C.c_int, [_P, C.c_int32]),
     "lbm_batch_lanes": (C.c_int, [_P]),
+    "lbm_batch_set_row_wait_limit": (C.c_int, [_P, C.c_int32]),
     "lbm_set_closure": (C.c_int, [_P, _P]),
     "lbm_set_closure_wait_limit": (C.c_int, [_P, C.c_int32]),
     "lbm_box_filter": (C.c_int, [_P, _P, _I32, _I32, _I32, _I32, _P, _P]),
@@ -443,6 +445,11 @@ class Lattice:
         """Whether step() streams rows through shared memory (lbm_step_streams_rows)."""
         return load().lbm_step_streams_rows(self._h) == 1
 
+    def set_row_wait_limit(self, polls: int) -> None:
+        """Testing hook: polls of a row-streaming step's wait for its copies (< 0:
+        the default, 0: give up at once); see lbm_set_row_wait_limit."""
+        self._c(load().lbm_set_row_wait_limit(self._h, int(polls)))
+
     def set_closure(self, net: np.ndarray | None) -> None:
         """Installs a learned-closure network (float[CLOSURE_FLOATS]); None
         removes it."""
@@ -608,6 +615,10 @@ class Batch:
     def lanes(self) -> int:
         """Parallel lanes that graph mode runs (lbm_batch_lanes)."""
         return load().lbm_batch_lanes(self._h)
+
+    def set_row_wait_limit(self, polls: int) -> None:
+        """Testing hook, as Lattice.set_row_wait_limit for every domain."""
+        self._c(load().lbm_batch_set_row_wait_limit(self._h, int(polls)))
 
     def info(self) -> BatchInfo:
         i = BatchInfo()

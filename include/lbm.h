@@ -211,6 +211,12 @@ LBM_API int lbm_set_step_variant(lbm_ctx* ctx, int nodes_per_thread);
  * < 0 on error. */
 LBM_API int lbm_step_streams_rows(lbm_ctx* ctx);
 
+/* Testing hook: bounds the wait of a step that streams rows for a tile's copies
+ * to `polls` polls (< 0: the default; 0: it gives up at once).  A step whose wait
+ * runs out stops in bounded time with its copies landed; lbm_sync reports
+ * LBM_ERR_TIMEOUT and the state needs a new init. */
+LBM_API int lbm_set_row_wait_limit(lbm_ctx* ctx, int32_t polls);
+
 /* The parameters in effect (from the descriptor, or the last lbm_set_params). */
 LBM_API int lbm_get_params(lbm_ctx* ctx, lbm_params* params);
 
@@ -512,6 +518,8 @@ LBM_API int lbm_batch_autotune(lbm_batch* b, int trial_steps, lbm_batch_schedule
  * side), 0 when it launches the tile kernel or the batch is in persistent mode;
  * < 0 on error. */
 LBM_API int lbm_batch_lanes(lbm_batch* b);
+/* lbm_set_row_wait_limit of every domain, for the lanes' steps. */
+LBM_API int lbm_batch_set_row_wait_limit(lbm_batch* b, int32_t polls);
 LBM_API int lbm_batch_get_info(lbm_batch* b, lbm_batch_info* info);
 LBM_API const char* lbm_batch_last_error(lbm_batch* b);
 
