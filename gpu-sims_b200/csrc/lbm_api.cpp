@@ -336,7 +336,7 @@ int lbm_set_step_variant(lbm_ctx* c, int nodes_per_thread) {
 int lbm_step_streams_rows(lbm_ctx* c) {
   if (int rc = check_ctx(c)) return rc;
   return c->d.mode == LBM_MODE_PHYSICS && c->step_variant == 0 && !c->closure &&
-         lbm::phys_rows_pay(c->pp.g, c->d.precision);
+         lbm::phys_rows_pay(c->pp, c->d);
 }
 
 int lbm_set_closure(lbm_ctx* c, const float* net) {

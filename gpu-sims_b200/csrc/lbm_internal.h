@@ -129,8 +129,8 @@ cudaError_t phys_rows_f16(const Ctx& c, int parity, bool write_moments, cudaStre
 cudaError_t phys_rows_bf16(const Ctx& c, int parity, bool write_moments, cudaStream_t s);
 // the number of its tiles for a grid, 0 where rows do not fit
 uint32_t phys_rows_tiles(const PhysGeom& g);
-// whether a lattice of this grid and precision takes it by default
-bool phys_rows_pay(const PhysGeom& g, int precision);
+// whether a lattice of these parameters (precision and collision of d) takes it by default
+bool phys_rows_pay(const PhysParams& p, const lbm_desc& d);
 cudaError_t phys_step_clo_f32(const Ctx& c, int parity, bool write_moments, cudaStream_t s);
 cudaError_t phys_step_clo_f16(const Ctx& c, int parity, bool write_moments, cudaStream_t s);
 cudaError_t phys_step_clo_bf16(const Ctx& c, int parity, bool write_moments, cudaStream_t s);

@@ -774,44 +774,73 @@ inline RowTiles row_tiles(const PhysGeom& G) {
   return rt;
 }
 
-// Row tiles (phys_rows.cuh) by default where rows fill their blocks and the
-// grid has enough tiles to fill the persistent blocks (148 or 296) several
-// times; else the row kernels' small blocks win.  The lines, measured on B200
-// (row tiles / row kernels, GLUPS):
-//  * rows below 66 nodes waste padding and tiles: 64^3 22.8 / 30.2 (fp16), 56 x
-//    56 x 200 29.5 / 36.2 (fp32), 57 x 57 x 200 26.0 / 31.0 (fp16);
-//  * nodes per 512-node tile: fp32 144^3 (0.84) 36.6 / 31.9, 200 x 97 x 120 (0.78)
-//    34.7 / 32.4, 385 x 97 x 120 (0.75) 32.9 / 31.4, 180 x 97 x 120 (0.70) 32.2 / 33.8,
-//    257 x 97 x 120 (0.50) 24.7 / 30.2; fp16 200 x 97 x 120 53.3 / 43.0, 192^3 (0.75)
-//    48.8 / 58.4, 320 x 97 x 120 (0.63) 54.9 / 56.5; odd rows, which only the one-node
-//    kernel takes otherwise, pay in 2-byte storage at any fill (257 43.3 / 35.1);
-//  * rows that leave the row kernels' 64-wide warps ragged: fp16 72^3 (792 tiles)
-//    27.2 / 23.4, fp32 72^3 24.2 / 24.2, 80^3 (1,120) 29.7 / 28.4;
-//  * rows of whole warps: fp16 128^3 (4,096) 56.1 / 55.6, 256 x 256 x 8 (1,024)
-//    45.1 / 51.9; fp32 256 x 128 x 128 (8,192) 37.8 / 38.3, 512 x 128 x 128 (16,384)
-//    41.2 / 39.4, 256^3 (32,768) 42.5 / 41.6.
-inline bool row_tiles_pay(const PhysGeom& G, int precision) {
-  const int nx = G.nx;
-  const RowTiles rt = row_tiles(G);
-  if (rt.R == 0 || nx < 66) return false;
-  const bool odd = nx % 2 != 0, whole = !odd && 20 * ((nx + 63) / 64 * 64) <= 23 * nx;
-  const int fill = 100 * rt.R * nx / 512;  // per cent of a tile
-  if (precision == LBM_PREC_F32) return fill >= 74 && rt.ntiles >= (whole ? 12000u : 1000u);
-  return (odd || fill >= 76) && rt.ntiles >= (whole ? 4000u : 700u);
-}
-
 // fp32 stages (45 KB) leave room for one block of five an SM or two of two.
 // Deep prefetch wins where the store streams from HBM (channel 512x128x128 41.6
 // against 38.6 GLUPS, cavity 160^3 37.6 against 34.4); where it stays in the
-// 126 MB L2, twice the consumer warps do (101^3 38.8 against 31.2, 161x97x75
-// with Smagorinsky 33.7 against 27.9, 96^3 38.2 against 29.8).
+// 126 MB L2, twice the consumer warps do (101^3 38.8 against 31.2, 96^3 38.2
+// against 29.8).  With Smagorinsky there is one block an SM in any case
+// (rows_blocks).
 constexpr size_t ROWS_DEEP_BYTES = 120000000;
 
+inline bool rows_deep(const PhysGeom& G, int precision, bool smag) {
+  return precision == LBM_PREC_F32 && (smag || 76 * G.slot_stride > ROWS_DEEP_BYTES);
+}
+// Persistent blocks of the chip's 148 SMs.
+inline uint32_t rows_chip_blocks(const PhysGeom& G, int precision, bool smag) {
+  return smag || rows_deep(G, precision, smag) ? 148 : 296;
+}
+
+// Where row tiles are the default: where they beat the row kernels
+// (phys_step_launch.cuh), measured on B200 over 56 row lengths from 66 to 512,
+// three sections and 26 thin boxes, both collisions, with and without
+// Smagorinsky, in graphs and in single steps (1,592 timings).  Ratios of the
+// two times, row tiles' to row kernels':
+//  * `used`, the share of the node slots of all blocks' rounds that hold nodes
+//    (tiles not filled by whole rows, a plane's ragged last tile, a last round of
+//    few blocks), decides most: odd rows in fp32 0.64-0.97 from 62 per cent on; with
+//    Smagorinsky, one block an SM, fp16 257 x 97 x 120 (50) 1.31, 181 x 97 x 120 (70)
+//    1.10, 97 x 140 x 140 (93) 0.81;
+//  * what it replaces: the pair kernels are at their best where rows fill their
+//    64-wide warps (`whole`), fp32 384 x 140 x 140 1.11, 512 x 140 x 140 0.95, fp16 with
+//    Smagorinsky 448 x 140 x 140 1.09, 112 x 140 x 140 0.87, 512 x 97 x 120 0.90; so is
+//    the one-node kernel, which odd rows with Smagorinsky take, at 32: 95 x 97 x 120
+//    1.12, 97 x 97 x 120 0.90;
+//  * tiles at a y face take twice the copies: one to three a plane 1.0-1.9, four
+//    of one row each 1.0-1.3, five of several rows 0.6-0.8; two planes of z 1.0-1.5;
+//  * few tiles: fp32 127 x 64 x 64 (1,024) 1.09, 67 x 300 x 24 (1,032) 0.76, fp16 75 x 64 x 64
+//    (704, 68 per cent used) 1.20, 71^3 (781, 79) 0.76, whole rows 256 x 256 x 8 (1,024) 1.15;
+//  * rows below 66 nodes waste padding and tiles: 64^3 fp16 22.8 against 30.2 GLUPS.
+// Open x faces cost the row kernels a launch of their own: 128^3 fp16 with
+// Smagorinsky 0.82, without the faces 1.03.  Inside the lines 1 in 50 of the
+// timings is slower by more than 4 per cent, the worst by 10 (81 x 97 x 120, periodic,
+// TRT, Smagorinsky, fp32, single steps).
+inline bool row_tiles_pay(const PhysParams& p, const lbm_desc& d) {
+  const PhysGeom& G = p.g;
+  const bool f32 = d.precision == LBM_PREC_F32, smag = p.smag_cs > 0.f, odd = G.nx % 2 != 0;
+  const RowTiles rt = row_tiles(G);
+  if (rt.R == 0 || G.nx < 66) return false;
+  const int wide = (G.nx + 63) / 64 * 64;
+  const bool whole = !odd && 20 * wide <= 23 * G.nx;
+  const int fill = 100 * rt.R * G.nx / 512;  // per cent of a tile
+  if (f32 ? fill < 74 : !odd && fill < 76) return false;
+  const uint32_t nt = rt.ntiles, blocks = rows_chip_blocks(G, d.precision, smag);
+  // per mille
+  const int used = (int)(1000 * (uint64_t)G.n / (512ull * blocks * ((nt + blocks - 1) / blocks)));
+  if (rt.tiles_y < (whole ? 12 : smag || rt.R < 5 ? 5 : 3)) return false;
+  if (G.nz < (smag && !odd ? 5 : 4) && !(odd && !f32 && !smag && used >= 750)) return false;
+  if (p.any_open) return nt >= (whole ? (f32 ? 12000u : 4000u) : (f32 ? 1000u : 700u));
+  if (whole)
+    return nt >= (f32 ? 12000u : 4000u) && used * wide >= G.nx * (f32 ? (smag ? 800 : 900) : (smag ? 920 : 720));
+  if (!smag) return nt >= (f32 ? 1030u : 700u) && used >= (f32 ? 620 : nt >= 1000 ? 450 : G.per[0] ? 660 : 750);
+  if (!odd) return nt >= (rt.R < 5 ? 1500u : 1030u) && used >= 700;
+  const bool many = nt >= (f32 ? 5000u : 2400u);
+  return nt >= 800 && used >= (many ? 720 : 800) &&
+         used * ((G.nx + 31) / 32 * 32) >= G.nx * (!many ? 880 : d.collision == LBM_COLL_TRT ? 870 : 800);
+}
 template <int PREC, int COLL, int SGS, bool FORCE, bool WM, bool OPEN>
 cudaError_t launch_row_tiles(const Ctx& c, int P, cudaStream_t s) {
   RowTiles rt = row_tiles(c.pp.g);
-  const bool deep = PREC == LBM_PREC_F32 && (SGS || 76 * c.pp.g.slot_stride > ROWS_DEEP_BYTES);
-  if (PREC == LBM_PREC_F32 && !deep) rt.stages = 2;
+  if (PREC == LBM_PREC_F32 && !rows_deep(c.pp.g, PREC, SGS)) rt.stages = 2;
   const size_t smem = (size_t)rt.stages * rows_stage<PREC>();
   auto* fn = &k_phys_rows<PREC, COLL, SGS, FORCE, WM, OPEN>;
   // The limit belongs to the kernel, which all lattices of the process share (other
@@ -820,7 +849,7 @@ cudaError_t launch_row_tiles(const Ctx& c, int P, cudaStream_t s) {
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        ROWS_MAXST * rows_stage<PREC>());
   if (e != cudaSuccess) return e;
-  const uint32_t most = c.row_blocks ? (uint32_t)c.row_blocks : 148u * (deep ? 1 : rows_blocks<PREC, SGS>());
+  const uint32_t most = c.row_blocks ? (uint32_t)c.row_blocks : rows_chip_blocks(c.pp.g, PREC, SGS);
   const dim3 grd(rt.ntiles < most ? rt.ntiles : most);
   fn<<<grd, ROWS_THREADS, smem, s>>>(c.pp, rt, c.pop, c.flags, c.links, c.rho, c.u, c.status, P, c.row_wait_polls);
   return cudaGetLastError();

@@ -8,5 +8,5 @@ uint32_t phys_rows_tiles(const PhysGeom& g) {
   const RowTiles rt = row_tiles(g);
   return rt.R ? rt.ntiles : 0;
 }
-bool phys_rows_pay(const PhysGeom& g, int precision) { return row_tiles_pay(g, precision); }
+bool phys_rows_pay(const PhysParams& p, const lbm_desc& d) { return row_tiles_pay(p, d); }
 }  // namespace lbm

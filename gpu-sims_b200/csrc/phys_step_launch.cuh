@@ -285,7 +285,7 @@ inline bool use_quads(const Ctx& c) {
   return c.step_variant == 4 || (c.step_variant == 0 && step_quads(nx));
 }
 inline bool use_row_tiles(const Ctx& c) {
-  return c.step_variant == 0 && !c.closure && row_tiles_pay(c.pp.g, c.d.precision);
+  return c.step_variant == 0 && !c.closure && row_tiles_pay(c.pp, c.d);
 }
 inline bool use_pairs(const Ctx& c) {
   const int nx = c.pp.g.nx;

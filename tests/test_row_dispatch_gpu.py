@@ -25,6 +25,46 @@ def test_choice_by_grid_variant_and_closure(gpu, prec):
     lat.close()
 
 
+SGS = {  # odd, ragged and whole rows with Smagorinsky
+    "odd": dict(shape=(97, 60, 355), cs=0.1, trt=True, lid=True),
+    "odd_periodic": dict(shape=(161, 51, 250), periodic=(1, 1, 1), cs=0.15, sphere=True),
+    "ragged": dict(shape=(72, 80, 160), periodic=(0, 1, 0), cs=0.1, lid=True, sphere=True),
+    "whole": dict(shape=(128, 120, 200), periodic=(1, 0, 0), cs=0.1, trt=True, sphere=True),
+}
+
+
+@pytest.mark.parametrize("prec,name", [(0, "odd"), (0, "odd_periodic"), (0, "ragged"), (1, "odd"), (1, "ragged"),
+                                       (1, "whole"), (2, "odd_periodic")])
+def test_smagorinsky(gpu, monkeypatch, prec, name):
+    case = SGS[name]
+    monkeypatch.setitem(CASES, "sgs", case)
+    lat = gpu.Lattice(nx=case["shape"][0], ny=case["shape"][1], nz=case["shape"][2], mode=gpu.MODE_PHYSICS,
+                      precision=prec, periodic=case.get("periodic", (0, 0, 0)), tau=0.57, smagorinsky_cs=case["cs"])
+    assert lat.streams_rows()
+    lat.set_params(smagorinsky_cs=0.0)  # the rule follows the parameters in effect
+    assert lat.streams_rows()
+    lat.close()
+    matches_one_node_kernel(gpu, prec, "sgs")
+
+
+def test_smagorinsky_changes_the_choice(gpu):
+    """257 x 97 x 20 in fp16: row tiles without the term (0.8 of the row kernels'
+    time), the row kernels with it (row tiles 1.3)."""
+    lat = gpu.Lattice(nx=257, ny=97, nz=20, mode=gpu.MODE_PHYSICS, precision=1, periodic=(1, 0, 0), tau=0.57)
+    assert lat.streams_rows()
+    lat.set_params(smagorinsky_cs=0.1)
+    assert not lat.streams_rows()
+    lat.close()
+
+
+@pytest.mark.parametrize("prec,shape", [(0, (512, 2, 2000)), (1, (512, 2, 2000)), (0, (129, 8000, 2)), (1, (129, 8000, 2)),
+                                        (0, (67, 3, 4000)), (1, (67, 3, 4000)), (0, (95, 4000, 3))])
+def test_thin_boxes_keep_the_row_kernels(gpu, prec, shape):
+    lat = gpu.Lattice(nx=shape[0], ny=shape[1], nz=shape[2], mode=gpu.MODE_PHYSICS, precision=prec, tau=0.57)
+    assert not lat.streams_rows()
+    lat.close()
+
+
 @pytest.mark.parametrize("case", [dict(shape=(160, 100, 100), lid=True, sphere=True),
                                   dict(shape=(161, 101, 101), periodic=(1, 0, 1), sphere=True, trt=True)])
 def test_five_stage_fp32(gpu, monkeypatch, case):

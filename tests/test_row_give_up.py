@@ -30,7 +30,7 @@ def moments(shape, seed):
 # two blocks an SM with two and with five stages, one block with five, no periodic axis and all
 @pytest.mark.gpu
 @pytest.mark.parametrize("prec,shape,per,cs", [(0, (101, 97, 64), (0, 0, 0), 0.0), (1, (97, 80, 80), (1, 1, 1), 0.0),
-                                               (2, (161, 60, 60), (0, 1, 0), 0.1), (0, (160, 100, 100), (1, 0, 0), 0.0)])
+                                               (2, (161, 60, 80), (0, 1, 0), 0.1), (0, (160, 100, 100), (1, 0, 0), 0.0)])
 def test_step_gives_up_and_recovers(gpu, prec, shape, per, cs):
     def lattice():
         lat = gpu.Lattice(nx=shape[0], ny=shape[1], nz=shape[2], mode=gpu.MODE_PHYSICS, precision=prec, periodic=per,
