@@ -434,16 +434,31 @@ int lbm_batch_create(const lbm_desc* descs, int n, lbm_batch** out) {
     v.d = descs[i];
     v.device = dev;
     v.n = (size_t)descs[i].nx * descs[i].ny * descs[i].nz;
-    if (!lbm::setup_physics(v, descs[i]))
-      return bail(bfail(b, LBM_ERR_UNSUPPORTED, "a domain exceeds 2^32 nodes per slot array"));
-    pop_off[i] = pop_total;
-    pop_total += up256(19 * v.pp.g.slot_stride * eb);
     aux_off[i] = aux_total;
     aux_total += up256(v.n) * 2 + up256(4 * v.n) * 2 + up256(12 * v.n);
     b->total_nodes += v.n;
   }
+  // periodic rows are padded for lanes where those are planned, and else, or
+  // where the padding does not fit, lie one behind the other
+  auto layout = [&](bool rows) {
+    pop_total = 0;
+    for (int i = 0; i < n; ++i) {
+      lbm::Ctx& v = b->dom[i];
+      if (!lbm::setup_physics(v, descs[i], rows)) return false;
+      pop_off[i] = pop_total;
+      pop_total += up256(19 * v.pp.g.slot_stride * eb);
+    }
+    plan_lanes(b);
+    return true;
+  };
   void *pop = nullptr, *aux = nullptr, *dd = nullptr, *st = nullptr;
-  if (int rc = balloc(b, &pop, pop_total, "cudaMalloc(population pool)")) return bail(rc);
+  const bool padded = layout(true) && !b->lanes.empty();
+  if (!padded && !layout(false))
+    return bail(bfail(b, LBM_ERR_UNSUPPORTED, "a domain exceeds 2^32 nodes per slot array"));
+  int pool_rc = balloc(b, &pop, pop_total, "cudaMalloc(population pool)");
+  if (pool_rc == LBM_ERR_OUT_OF_MEMORY && padded && layout(false))
+    pool_rc = balloc(b, &pop, pop_total, "cudaMalloc(population pool)");
+  if (pool_rc) return bail(pool_rc);
   if (int rc = balloc(b, &aux, aux_total, "cudaMalloc(aux pool)")) return bail(rc);
   if (int rc = balloc(b, &dd, n * sizeof(lbm::BatchDomain), "cudaMalloc(tile table)")) return bail(rc);
   if (int rc = balloc(b, &st, 256, "cudaMalloc(status)")) return bail(rc);
@@ -472,7 +487,6 @@ int lbm_batch_create(const lbm_desc* descs, int n, lbm_batch** out) {
     const int per[3] = {v.d.periodic[0], v.d.periodic[1], v.d.periodic[2]};
     if (cudaError_t e = lbm::classify(v, per, b->stream)) return bail(bcuda(b, e, "classify"));
   }
-  plan_lanes(b);
   if (int rc = build_tiles(b)) return bail(rc);
   *out = b;
   return LBM_OK;

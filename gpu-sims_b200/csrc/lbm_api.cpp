@@ -149,12 +149,12 @@ namespace lbm {
 
 void set_thread_error(const char* msg) { g_thread_err = msg; }
 
-bool setup_physics(Ctx& c, const lbm_desc& d) {
+bool setup_physics(Ctx& c, const lbm_desc& d, bool rows) {
   auto& g = c.pp.g;
   g.nx = d.nx; g.ny = d.ny; g.nz = d.nz;
   g.n = (size_t)d.nx * d.ny * d.nz;
   for (int a = 0; a < 3; ++a) g.per[a] = d.periodic[a];
-  g.px = (int)round_up((size_t)g.nx + (g.per[0] ? 0 : 1), 8);
+  g.px = g.per[0] && !rows ? g.nx : (int)round_up((size_t)g.nx + (g.per[0] ? 0 : 1), 8);
   g.gy = g.per[1] ? 0 : 1;
   g.gz = g.per[2] ? 0 : 1;
   g.py = g.ny + 2 * g.gy;
@@ -262,12 +262,24 @@ int lbm_create(const lbm_desc* desc, lbm_ctx** out) {
     p.free_slip = desc->ref_free_slip;
     p.u_round = desc->ref_u_round;
   } else {
-    if (!lbm::setup_physics(*c, *desc))
-      return bail(fail(c, LBM_ERR_UNSUPPORTED, "padded grid exceeds 2^32 nodes per slot array"));
+    // periodic rows are padded for the row tiles where those may run (lbm_set_params
+    // can turn Smagorinsky on and off), and else, or where the padding does not fit,
+    // lie one behind the other
     const size_t eb = lbm::elem_bytes(desc->precision);
-    if ((rc = dev_alloc(c, reinterpret_cast<char**>(&c->pop), 19 * c->pp.g.slot_stride * eb,
-                        "cudaMalloc(populations)")))
-      return bail(rc);
+    bool rows = lbm::setup_physics(*c, *desc, true);
+    if (rows) {
+      lbm::PhysParams plain = c->pp, smag = c->pp;
+      plain.smag_cs = 0.f;
+      smag.smag_cs = 0.1f;
+      rows = lbm::phys_rows_pay(plain, *desc) || lbm::phys_rows_pay(smag, *desc);
+    }
+    for (;; rows = false) {
+      if (!rows && !lbm::setup_physics(*c, *desc, false))
+        return bail(fail(c, LBM_ERR_UNSUPPORTED, "padded grid exceeds 2^32 nodes per slot array"));
+      rc = dev_alloc(c, reinterpret_cast<char**>(&c->pop), 19 * c->pp.g.slot_stride * eb, "cudaMalloc(populations)");
+      if (!rc) break;
+      if (!rows || !desc->periodic[0] || rc != LBM_ERR_OUT_OF_MEMORY) return bail(rc);
+    }
   }
   c->nblk_cons = lbm::cons_blocks(n);
   if ((rc = dev_alloc(c, &c->mask, n, "cudaMalloc(mask)")) ||
@@ -802,7 +814,7 @@ int lbm_set_params(lbm_ctx* c, const lbm_params* p) {
       if (e != cudaSuccess) return cuda_fail(c, e, "recompute collision");
     }
   } else {
-    lbm::setup_physics(*c, d);
+    lbm::setup_physics(*c, d, c->pp.g.px > d.nx);  // the layout stays
   }
   return c->initialized ? prepare_graphs(c) : LBM_OK;
 }

@@ -208,7 +208,8 @@ size_t elem_bytes(int precision);
 float round_bf16(float v);
 // Fills c.pp (padded geometry and physics parameters) from a physics-mode
 // descriptor; false if a slot array would exceed 2^32 elements.
-bool setup_physics(Ctx& c, const lbm_desc& d);
+// rows: periodic rows padded to 8 elements, as the row tiles need them
+bool setup_physics(Ctx& c, const lbm_desc& d, bool rows);
 int validate_desc(const lbm_desc* d);
 // NACA perimeter of lbm_voxelize_naca in lattice units (x0 y0 x1 y1 ...);
 // false for a designation that is not four digits (host_tools.cpp).

@@ -757,10 +757,11 @@ __global__ void __launch_bounds__(ROWS_THREADS, rows_blocks<PREC, SGS>())
   });
 }
 
-// Tiles of a grid; R = 0 when a row does not fit.
+// Tiles of a grid; R = 0 when a row does not fit or its copies would not start
+// on 16-byte boundaries.
 inline RowTiles row_tiles(const PhysGeom& G) {
   RowTiles rt{};
-  if (G.nx < 4 || G.px > ROWS_CAP || (uint64_t)Q * G.slot_stride * 4 >= ROWS_MOST_BYTES) return rt;
+  if (G.nx < 4 || G.px % 8 || G.px > ROWS_CAP || (uint64_t)Q * G.slot_stride * 4 >= ROWS_MOST_BYTES) return rt;
   rt.tpr = (G.nx + 1) / 2;
   if (rt.tpr > ROWS_CONS) return rt;
   int R = ROWS_CAP / G.px;
@@ -781,7 +782,6 @@ inline RowTiles row_tiles(const PhysGeom& G) {
 // against 29.8).  With Smagorinsky there is one block an SM in any case
 // (rows_blocks).
 constexpr size_t ROWS_DEEP_BYTES = 120000000;
-
 inline bool rows_deep(const PhysGeom& G, int precision, bool smag) {
   return precision == LBM_PREC_F32 && (smag || 76 * G.slot_stride > ROWS_DEEP_BYTES);
 }
@@ -837,6 +837,7 @@ inline bool row_tiles_pay(const PhysParams& p, const lbm_desc& d) {
   return nt >= 800 && used >= (many ? 720 : 800) &&
          used * ((G.nx + 31) / 32 * 32) >= G.nx * (!many ? 880 : d.collision == LBM_COLL_TRT ? 870 : 800);
 }
+
 template <int PREC, int COLL, int SGS, bool FORCE, bool WM, bool OPEN>
 cudaError_t launch_row_tiles(const Ctx& c, int P, cudaStream_t s) {
   RowTiles rt = row_tiles(c.pp.g);
