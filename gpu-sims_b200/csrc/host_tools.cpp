@@ -10,6 +10,7 @@
 
 #include "../../include/lbm.h"
 #include "d3q19.cuh"
+#include "colormap.h"
 #include "lbm_internal.h"
 
 namespace {
@@ -213,28 +214,11 @@ const char* lbm_build_info(void) {
 // to bytes.
 extern "C" int lbm_colormap_lut(uint8_t* out) {
   if (!out) return LBM_ERR_INVALID_ARG;
-  auto clamp01 = [](float v) { return v < 0.0f ? 0.0f : (v > 1.0f ? 1.0f : v); };
   for (int i = 0; i < 256; ++i) {
-    const float t = (float)i / 255.0f;
-    float r, g, b;
-    if (t < 0.25f) {
-      const float f = t / 0.25f;
-      r = 0.05f; g = 0.05f + 0.6f * f; b = 0.4f + 0.6f * f;
-    } else if (t < 0.5f) {
-      const float f = (t - 0.25f) / 0.25f;
-      r = 0.05f; g = 0.65f + 0.3f * f; b = 1.0f - 0.7f * f;
-    } else if (t < 0.75f) {
-      const float f = (t - 0.5f) / 0.25f;
-      r = 0.05f + 0.95f * f; g = 0.95f - 0.05f * f; b = 0.3f - 0.25f * f;
-    } else {
-      const float f = (t - 0.75f) / 0.25f;
-      r = 1.0f; g = 0.9f - 0.7f * f; b = 0.05f;
-    }
-    const uint8_t rgb[3] = {(uint8_t)(clamp01(r) * 255.0f), (uint8_t)(clamp01(g) * 255.0f),
-                            (uint8_t)(clamp01(b) * 255.0f)};
+    const lbm::ColormapEntry e = lbm::colormap_entry(i);
     for (int row = 0; row < 4; ++row) {
       uint8_t* o = out + 4 * (row * 256 + i);
-      o[0] = rgb[0]; o[1] = rgb[1]; o[2] = rgb[2]; o[3] = 255;
+      o[0] = e.rgb[0]; o[1] = e.rgb[1]; o[2] = e.rgb[2]; o[3] = 255;
     }
   }
   return LBM_OK;

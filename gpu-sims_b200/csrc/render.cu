@@ -1,5 +1,5 @@
-// Velocity-magnitude volume raymarch into a headless RGBA buffer: two lanes per
-// pixel.  Restates the reference's velmag fragment pass (volumetric-grid/
+// Velocity-magnitude volume raymarch into a headless RGBA buffer: one or two
+// lanes per pixel.  Restates the reference's velmag fragment pass (volumetric-grid/
 // lattice-boltzmann/shaders/velmag.frag.glsl:44-96, uniforms from
 // src/main.cpp:1720-1731, LUTs src/main.cpp:529-573, full-screen triangle
 // shaders/fullscreen.vert.glsl) without a graphics API: no swapchain,
@@ -23,6 +23,7 @@
 #include <string>
 #include <type_traits>
 
+#include "colormap.h"
 #include "lbm_internal.h"
 
 namespace lbm {
@@ -36,8 +37,21 @@ struct RenderArgs {
   float absorption, mag_min, mag_max, exposure;
   int width, height;
   float inv_ext[3];   // 1 / extent where the extent is a power of two, else 0
-  unsigned char lut[256][3];  // colour LUT row (rgb bytes)
 };
+
+// The colour table as the shader samples it: bytes / 255, divided at compile time.
+struct ColorTable {
+  float4 e[256];
+};
+constexpr ColorTable color_table() {
+  ColorTable t{};
+  for (int i = 0; i < 256; ++i) {
+    const ColormapEntry c = colormap_entry(i);
+    t.e[i] = float4{(float)c.rgb[0] / 255.0f, (float)c.rgb[1] / 255.0f, (float)c.rgb[2] / 255.0f, 0.0f};
+  }
+  return t;
+}
+__device__ const ColorTable COLORS = color_table();
 
 __device__ __forceinline__ float mul(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ float add(float a, float b) { return __fadd_rn(a, b); }
@@ -122,32 +136,32 @@ __device__ __forceinline__ void sample_u(const Vol<I, F16>& V, float cx, float c
   }
 }
 
-// Two lanes a ray.  A sample is some 400 dependent instructions and a ray up to
-// `steps` of them in sequence, so with a lane a ray the image waits for its
-// longest rays; the samples themselves do not depend on each other.  Lane l takes
-// samples l, l + 2, ... (its t by the same additions), and a ray's lanes
-// composite each group in order from one another's colours, with the same
+// One or two lanes a ray (two_lanes).  A sample is some 400 dependent instructions
+// and a ray up to `steps` of them in sequence, so with a lane a ray the image waits
+// for its longest rays; the samples themselves do not depend on each other.  Of
+// two lanes each takes every other sample (its t by the same additions), and they
+// composite each pair in order from one another's colours, with the same
 // operations as one lane alone.  More lanes spend the gain on samples beyond the
-// end of rays that saturate early.  B200, 1280 x 720 over 128^3, 128 steps,
-// 1 / 2 / 4 lanes: image 350 / 290 / 292 us, a whole viewer frame by itself 648 /
-// 585 / 588, frames of several viewers one behind the other 412 / 425 / 476 (702 and
-// 467 before).
+// end of rays that saturate early: 1280 x 720 over 128^3, 128 steps, 1 / 2 / 4 lanes:
+// 350 / 290 / 292 us.
 //
-// The colour table lies in shared memory, already divided by 255: the rays of
-// a warp read different entries, which kernel parameter space serves one after
-// the other, and six divisions a sample gave the same 768 values (one lane a ray:
-// 415 -> 350 us).  An extent that is a power of two divides by an exact product.
-constexpr int RAY_LANES = 2;
-constexpr int TILE_X = 8, TILE_Y = 32 / RAY_LANES;  // pixels of a block of 256 threads
+// The colour table lies in shared memory: the rays of a warp read different
+// entries, which kernel parameter space serves one after the other (one lane a
+// ray: 415 -> 350 us).  A block copies it from global memory, where it lies divided
+// by 255 at compile time; making it from kernel parameters in every block took
+// 70 us of a 1920 x 1080 image of any length (1 step 120 -> 35 us).  Blocks that no
+// ray of theirs enters the volume from stop there.  An extent that is a power of
+// two divides by an exact product.
+constexpr int TILE_X = 8;
+template <int RAY_LANES> constexpr int tile_y() { return 32 / RAY_LANES; }  // pixels of a block of 256 threads
 
-template <class I, bool F16>
-__global__ void __launch_bounds__(TILE_X * TILE_Y * RAY_LANES)
+template <class I, bool F16, int RAY_LANES>
+__global__ void __launch_bounds__(256)
     k_velmag(Vol<I, F16> V, const __grid_constant__ RenderArgs R, float4* __restrict__ out) {
   __shared__ float4 lut[256];
+  constexpr int TILE_Y = tile_y<RAY_LANES>();
   static_assert(TILE_X * TILE_Y * RAY_LANES == 256, "one table entry a thread");
-  lut[threadIdx.x] = make_float4(dv((float)R.lut[threadIdx.x][0], 255.0f), dv((float)R.lut[threadIdx.x][1], 255.0f),
-                                 dv((float)R.lut[threadIdx.x][2], 255.0f), 0.0f);
-  __syncthreads();
+  lut[threadIdx.x] = COLORS.e[threadIdx.x];
   const int q = threadIdx.x / RAY_LANES, l = threadIdx.x % RAY_LANES;
   const unsigned tiles_x = (unsigned)(R.width + TILE_X - 1) / TILE_X;
   const int px = (int)(blockIdx.x % tiles_x) * TILE_X + q % TILE_X;
@@ -176,6 +190,10 @@ __global__ void __launch_bounds__(TILE_X * TILE_Y * RAY_LANES)
   const bool hit = pixel && !(tx < te || tx < 0.0f);
   const float t0 = fmaxf(te, 0.0f);
   const float ray = sub(tx, t0);
+  if (!__syncthreads_or(hit)) {  // also: the table is complete
+    if (pixel && l == 0) out[(size_t)py * R.width + px] = make_float4(0.f, 0.f, 0.f, 0.f);
+    return;
+  }
   float jitter = 0.0f;
   if (hit) {
     const unsigned jx = px > 255 ? 255u : (unsigned)px, jy = py > 255 ? 255u : (unsigned)py;
@@ -240,6 +258,14 @@ __global__ void __launch_bounds__(TILE_X * TILE_Y * RAY_LANES)
                                          : make_float4(0.f, 0.f, 0.f, 0.f);
 }
 
+// Two lanes a ray for the samples of long rays, and for images of fewer pixels than
+// the chip's resident threads.  B200, 1 / 2 lanes in us: 1920 x 1080 over 256 x 128 x
+// 128, absorption 5: 1 step 25 / 50, 8 steps 30 / 50, 24 48 / 54, 32 59 / 58, 128 179 /
+// 128; 320 x 200 over 128^3: 1 step 8.2 / 7.9, 4 8.8 / 9.2, 8 13 / 11, 32 35 / 21.
+inline bool two_lanes(int steps, int width, int height) {
+  return steps >= 24 || (steps >= 4 && (int64_t)width * height < 148 * 1024);
+}
+
 }  // namespace
 }  // namespace lbm
 
@@ -289,25 +315,25 @@ int lbm_render_velmag(const float* d_u, int32_t nx, int32_t ny, int32_t nz, cons
   R.exposure = p->exposure;
   R.width = width;
   R.height = height;
-  unsigned char lut[256 * 4 * 4];
-  lbm_colormap_lut(lut);
-  for (int i = 0; i < 256; ++i)
-    for (int c = 0; c < 3; ++c) R.lut[i][c] = lut[4 * i + c];  // row 0 (all rows equal)
   for (int c = 0; c < 3; ++c) {
     int ex = 0;
     const float ext = R.vmax[c] - R.vmin[c];
     R.inv_ext[c] = std::frexp(ext, &ex) == 0.5f && ex > -100 && ex < 100 ? 1.0f / ext : 0.0f;
   }
   const size_t n = (size_t)nx * ny * nz;
-  const dim3 blk(lbm::TILE_X * lbm::TILE_Y * lbm::RAY_LANES);
-  const unsigned grd = (unsigned)((width + lbm::TILE_X - 1) / lbm::TILE_X) *
-                       (unsigned)((height + lbm::TILE_Y - 1) / lbm::TILE_Y);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   float4* out = reinterpret_cast<float4*>(d_rgba);
-  auto launch = [&](auto index, auto f16) {
+  auto lanes = [&](auto index, auto f16, auto ray) {
     using I = decltype(index);
     constexpr bool F16 = decltype(f16)::value;
-    lbm::k_velmag<I, F16><<<grd, blk, 0, s>>>(lbm::Vol<I, F16>{d_u, nx, ny, nz, n}, R, out);
+    constexpr int L = decltype(ray)::value, TY = lbm::tile_y<L>();
+    const unsigned grd =
+        (unsigned)((width + lbm::TILE_X - 1) / lbm::TILE_X) * (unsigned)((height + TY - 1) / TY);
+    lbm::k_velmag<I, F16, L><<<grd, 256, 0, s>>>(lbm::Vol<I, F16>{d_u, nx, ny, nz, n}, R, out);
+  };
+  auto launch = [&](auto index, auto f16) {
+    if (lbm::two_lanes(p->steps, width, height)) lanes(index, f16, std::integral_constant<int, 2>{});
+    else lanes(index, f16, std::integral_constant<int, 1>{});
   };
   if (n < (1u << 31)) {
     if (p->round_f16) launch(uint32_t{}, std::true_type{});
