@@ -250,11 +250,10 @@ __global__ void __launch_bounds__(256) k_predict(const float* __restrict__ net,
 // its share of the rest, each summing the 32 samples with no atomics.  At the
 // end the block's gradient goes to its row of `part`, which the Adam kernel sums
 // over blocks in a fixed order: the gradient is deterministic.
-// Bound by the latency of its sums at the batch sizes of training, by shared
-// loads beyond: a warp that took 32 samples by itself needed 3,900 steps for them
-// one after the other (batch of 4,096: 16.6 us on 32 SMs, and 6.2 us to sum over
-// blocks).  lbm_trainer_grad, gradient read back: 4,096 samples 46.8 -> 33.6 us,
-// 65,536 77 -> 62, 300,000 139 -> 139.
+// Bound by the latency of its sums at the batch sizes of training: a warp that
+// takes 32 samples by itself (k_mlp_grad_wide) needs 3,900 steps for them one after
+// the other (batch of 4,096: 16.6 us on 32 SMs, and 6.2 us to sum over blocks).
+// lbm_trainer_grad, gradient read back, 4,096 samples: 46.8 -> 33.6 us.
 // Sample j of the batch is dataset row (a * (start + j) + c) mod n.
 // ---------------------------------------------------------------------------
 constexpr int TR_WARPS = 4;
@@ -463,6 +462,197 @@ __global__ void __launch_bounds__(TR_THREADS, 4)
   }
 }
 
+// The same for large batches: a warp takes 32 samples at a time by itself, lane =
+// sample, the activations in registers, and leaves them and the pre-activation
+// gradients in its own tiles for the weight gradients (lane = hidden unit i: row
+// i of dW2 and dW1), which the block's warps add in order at the end.  A sample
+// costs fewer shared loads than in k_mlp_grad, and with all SMs busy the length
+// of a warp's chain no longer shows.  An optimiser step with batches of 16,384
+// samples takes 26.5 us by k_mlp_grad and 27.4 by this one, of 32,768 36.4 and 29.3,
+// 65,536 49.9 and 41.6, 262,144 134 and 105, 1,200,000 520 and 410; lbm_trainer_grad
+// of 16,384 43.6 and 52.0, of 32,768 52.0 and 50.8: hence TR_WIDE.
+constexpr int64_t TR_WIDE = 24576;
+constexpr int TRW_MAX_BLOCKS = 296;  // two per SM
+constexpr int TRW_WARP_FLOATS = 4 * 32 * TR_LD + 32 * TR_XLD + 32;
+constexpr size_t TRW_SMEM = (size_t)(TR_NET + CLO_HID * CLO_HID + TR_WARPS * TRW_WARP_FLOATS) * 4;
+static_assert(TRW_WARP_FLOATS % 4 == 0 && CLO_NPARAM <= TRW_WARP_FLOATS && TRW_MAX_BLOCKS <= TR_MAX_BLOCKS,
+              "float4 tiles; a warp's gradient row fits them");
+
+__global__ void __launch_bounds__(TR_THREADS, 2)
+    k_mlp_grad_wide(const float* __restrict__ net, Batch B, float* __restrict__ part,
+                    double* __restrict__ loss_part) {
+  extern __shared__ __align__(16) float sm[];
+  float* sw = sm;                                       // network [CLO_FLOATS] (padded)
+  float* sW2T = sm + TR_NET;                            // W2 transposed [j][i]
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  float* wb = sW2T + CLO_HID * CLO_HID + warp * TRW_WARP_FLOATS;
+  float* sH1 = wb;                  // [32][TR_LD] h1 per sample
+  float* sH2 = sH1 + 32 * TR_LD;    // h2
+  float* sA1 = sH2 + 32 * TR_LD;    // d a1
+  float* sA2 = sA1 + 32 * TR_LD;    // d a2
+  float* sX = sA2 + 32 * TR_LD;     // [32][TR_XLD] standardised inputs
+  float* sDZ = sX + 32 * TR_XLD;    // [32] d z
+
+  for (int k = threadIdx.x; k < CLO_FLOATS; k += TR_THREADS) sw[k] = net[k];
+  for (int k = threadIdx.x; k < CLO_HID * CLO_HID; k += TR_THREADS) {
+    const int i = k / CLO_HID, j = k % CLO_HID;
+    sW2T[j * CLO_HID + i] = net[CLO_W2 + k];
+  }
+  __syncthreads();
+
+  float gW2[CLO_HID], gW1[CLO_IN];
+#pragma unroll
+  for (int j = 0; j < CLO_HID; ++j) gW2[j] = 0.f;
+#pragma unroll
+  for (int k = 0; k < CLO_IN; ++k) gW1[k] = 0.f;
+  float gb1 = 0.f, gb2 = 0.f, gW3 = 0.f, gb3 = 0.f;
+  double lsum = 0.0;
+
+  const int64_t groups = (B.nb + 31) / 32;
+  for (int64_t gi = (int64_t)blockIdx.x * TR_WARPS + warp; gi < groups;
+       gi += (int64_t)gridDim.x * TR_WARPS) {
+    // ---- forward and activation backward, lane = sample ----
+    const int64_t j = gi * 32 + lane;
+    const bool valid = j < B.nb;
+    float xs[CLO_IN];
+    float tgt = 0.f, wt = 0.f;
+    if (valid) {
+      const uint64_t pos = (uint64_t)(B.start + j);
+      const size_t row = (size_t)((B.a * pos + B.c) % (uint64_t)B.n);
+#pragma unroll
+      for (int k = 0; k < CLO_IN; ++k)
+        xs[k] = (B.x[row * CLO_IN + k] - sw[CLO_MEAN + k]) * sw[CLO_ISCALE + k];
+      tgt = B.t[row];
+      wt = B.w[row];
+    } else {
+#pragma unroll
+      for (int k = 0; k < CLO_IN; ++k) xs[k] = 0.f;
+    }
+    float h1[CLO_HID];
+#pragma unroll
+    for (int i = 0; i < CLO_HID; ++i) {
+      float a = sw[CLO_B1 + i];
+#pragma unroll
+      for (int k = 0; k < CLO_IN; ++k) a = fmaf(sw[CLO_W1 + i * CLO_IN + k], xs[k], a);
+      h1[i] = fmaxf(a, 0.f);
+    }
+    float z = sw[CLO_B3];
+    unsigned m2 = 0;
+#pragma unroll
+    for (int i = 0; i < CLO_HID; i += 4) {
+      float h2v[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const float4* wr = reinterpret_cast<const float4*>(sw + CLO_W2 + (i + q) * CLO_HID);
+        float a = sw[CLO_B2 + i + q];
+#pragma unroll
+        for (int jj = 0; jj < CLO_HID / 4; ++jj) {
+          const float4 w4 = wr[jj];
+          a = fmaf(w4.x, h1[4 * jj], a);
+          a = fmaf(w4.y, h1[4 * jj + 1], a);
+          a = fmaf(w4.z, h1[4 * jj + 2], a);
+          a = fmaf(w4.w, h1[4 * jj + 3], a);
+        }
+        h2v[q] = fmaxf(a, 0.f);
+        if (a > 0.f) m2 |= 1u << (i + q);
+        z = fmaf(sw[CLO_W3 + i + q], h2v[q], z);
+      }
+      *reinterpret_cast<float4*>(sH2 + lane * TR_LD + i) = make_float4(h2v[0], h2v[1], h2v[2], h2v[3]);
+    }
+#pragma unroll
+    for (int i = 0; i < CLO_HID; i += 4)
+      *reinterpret_cast<float4*>(sH1 + lane * TR_LD + i) = make_float4(h1[i], h1[i + 1], h1[i + 2], h1[i + 3]);
+    // softplus output and the weighted squared error
+    const float r = z > 20.f ? z : log1pf(expf(z));
+    const float sig = 1.f / (1.f + expf(-z));
+    const float e = r - tgt;
+    const float dz = valid ? 2.f * B.wscale * wt * e * sig : 0.f;
+    if (valid) lsum += (double)B.wscale * (double)wt * (double)e * (double)e;
+    float da2[CLO_HID];
+#pragma unroll
+    for (int i = 0; i < CLO_HID; ++i) da2[i] = (m2 >> i & 1u) ? sw[CLO_W3 + i] * dz : 0.f;
+#pragma unroll
+    for (int i = 0; i < CLO_HID; i += 4)
+      *reinterpret_cast<float4*>(sA2 + lane * TR_LD + i) = make_float4(da2[i], da2[i + 1], da2[i + 2], da2[i + 3]);
+    // d a1_j = [a1_j > 0] sum_i W2[i][j] d a2_i  (W2 transposed: row j contiguous)
+#pragma unroll
+    for (int jq = 0; jq < CLO_HID; jq += 4) {
+      float d[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int jj = jq + q;
+        const float4* wr = reinterpret_cast<const float4*>(sW2T + jj * CLO_HID);
+        float a = 0.f;
+#pragma unroll
+        for (int i4 = 0; i4 < CLO_HID / 4; ++i4) {
+          const float4 w4 = wr[i4];
+          a = fmaf(w4.x, da2[4 * i4], a);
+          a = fmaf(w4.y, da2[4 * i4 + 1], a);
+          a = fmaf(w4.z, da2[4 * i4 + 2], a);
+          a = fmaf(w4.w, da2[4 * i4 + 3], a);
+        }
+        d[q] = h1[jj] > 0.f ? a : 0.f;
+      }
+      *reinterpret_cast<float4*>(sA1 + lane * TR_LD + jq) = make_float4(d[0], d[1], d[2], d[3]);
+    }
+#pragma unroll
+    for (int k = 0; k < CLO_IN; ++k) sX[lane * TR_XLD + k] = xs[k];
+    sDZ[lane] = dz;
+    __syncwarp();
+    // ---- weight gradients, lane = hidden unit ----
+    for (int s = 0; s < 32; ++s) {
+      const float a2 = sA2[s * TR_LD + lane];
+      const float a1 = sA1[s * TR_LD + lane];
+      const float dzs = sDZ[s];
+      const float4* h = reinterpret_cast<const float4*>(sH1 + s * TR_LD);
+#pragma unroll
+      for (int q = 0; q < CLO_HID / 4; ++q) {
+        const float4 hv = h[q];
+        gW2[4 * q] = fmaf(a2, hv.x, gW2[4 * q]);
+        gW2[4 * q + 1] = fmaf(a2, hv.y, gW2[4 * q + 1]);
+        gW2[4 * q + 2] = fmaf(a2, hv.z, gW2[4 * q + 2]);
+        gW2[4 * q + 3] = fmaf(a2, hv.w, gW2[4 * q + 3]);
+      }
+#pragma unroll
+      for (int k = 0; k < CLO_IN; ++k) gW1[k] = fmaf(a1, sX[s * TR_XLD + k], gW1[k]);
+      gb1 += a1;
+      gb2 += a2;
+      gW3 = fmaf(dzs, sH2[s * TR_LD + lane], gW3);
+      gb3 += dzs;
+    }
+    __syncwarp();
+  }
+
+  // ---- block reduction in a fixed order ----
+  // loss: warp sum (butterfly, the same order on every run), then warps in order
+  for (int o = 16; o > 0; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
+  __syncthreads();  // every warp is done with its tiles
+  float* g = wb;    // this warp's gradient row, CLO_NPARAM floats (fits the tiles)
+#pragma unroll
+  for (int jj = 0; jj < CLO_HID; ++jj) g[CLO_W2 + lane * CLO_HID + jj] = gW2[jj];
+#pragma unroll
+  for (int k = 0; k < CLO_IN; ++k) g[CLO_W1 + lane * CLO_IN + k] = gW1[k];
+  g[CLO_B1 + lane] = gb1;
+  g[CLO_B2 + lane] = gb2;
+  g[CLO_W3 + lane] = gW3;
+  if (lane == 0) g[CLO_B3] = gb3;
+  __shared__ double sl[TR_WARPS];
+  if (lane == 0) sl[warp] = lsum;
+  __syncthreads();
+  const float* g0 = sW2T + CLO_HID * CLO_HID;
+  for (int k = threadIdx.x; k < CLO_NPARAM; k += TR_THREADS) {
+    float acc = g0[k];
+#pragma unroll
+    for (int w = 1; w < TR_WARPS; ++w) acc += g0[w * TRW_WARP_FLOATS + k];
+    part[(size_t)blockIdx.x * CLO_NPARAM + k] = acc;
+  }
+  if (threadIdx.x == 0) {
+    double l = 0.0;
+    for (int w = 0; w < TR_WARPS; ++w) l += sl[w];
+    loss_part[blockIdx.x] = l;
+  }
+}
+
 struct AdamArgs {
   float lr, b1, b2, eps, wd;
   float bc1, bc2;   // 1 - beta^t
@@ -579,14 +769,23 @@ int tcuda(lbm_trainer* t, cudaError_t e, const char* what) {
     if (e_ != cudaSuccess) return tcuda(t, e_, what);   \
   } while (0)
 
-int grid_for(int64_t nb) {
-  const int64_t blocks = (nb + 31) / 32;
-  return (int)(blocks < 1 ? 1 : blocks > TR_MAX_BLOCKS ? TR_MAX_BLOCKS : blocks);
+// blocks for nb samples, `each` of them a block, `most` blocks at the most
+int grid_for(int64_t nb, int64_t each, int most) {
+  const int64_t blocks = (nb + each - 1) / each;
+  return (int)(blocks < 1 ? 1 : blocks > most ? most : blocks);
 }
 
 int launch_grad(lbm_trainer* t, const Batch& B, int* nblk) {
-  const int g = grid_for(B.nb);
-  k_mlp_grad<<<g, TR_THREADS, 0, t->stream>>>(t->net, B, t->part, t->loss_part);
+  int g;
+  if (B.nb < TR_WIDE) {
+    g = grid_for(B.nb, 32, TR_MAX_BLOCKS);
+    k_mlp_grad<<<g, TR_THREADS, 0, t->stream>>>(t->net, B, t->part, t->loss_part);
+  } else {
+    g = grid_for(B.nb, 32 * TR_WARPS, TRW_MAX_BLOCKS);
+    TCK(t, cudaFuncSetAttribute(k_mlp_grad_wide, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TRW_SMEM),
+        "closure grad kernel attribute");
+    k_mlp_grad_wide<<<g, TR_THREADS, TRW_SMEM, t->stream>>>(t->net, B, t->part, t->loss_part);
+  }
   TCK(t, cudaGetLastError(), "closure grad kernel");
   *nblk = g;
   return LBM_OK;
