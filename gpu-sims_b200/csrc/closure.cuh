@@ -19,18 +19,21 @@
 
 namespace lbm {
 
-// Network handed to a step kernel by value: biases, input scaling and the
-// weights of kernels that run a layer on CUDA cores are constant-bank operands;
-// the matrix products read their fragments from `frag`.  Kernels without the
-// closure take the one-float placeholder.
+// Network handed to a step kernel by value: what the warp-level matrix products
+// do not read from their fragments, so that a launch and a graph's node carry 88
+// bytes and not the 5.7 KB of the whole network.  Kernels without the closure
+// take the one-float placeholder.
 template <int SGS> struct CloNet {
   float v[1];
-  __device__ __forceinline__ float operator[](int) const { return 0.0f; }
 };
 template <> struct CloNet<2> {
-  float v[CLO_FLOATS];
+  float mean[CLO_IN], iscale[CLO_IN], b3;
   const uint4* frag;  // device: the layers as matrix fragments (clo_fragments)
-  __device__ __forceinline__ float operator[](int k) const { return v[k]; }
+};
+// The whole network by value: every weight a constant-bank operand (the tcgen05
+// kernel builds its tiles from it).
+struct CloFull {
+  float v[CLO_FLOATS];
 };
 
 // SGS 3: the same network with its hidden layer on the tensor cores.  One
@@ -52,7 +55,7 @@ template <> struct CloNet<2> {
 // MMA and falls back to r = 1, and the kernel drains the last commit (again
 // bounded) before it frees its tensor memory.
 template <> struct CloNet<3> {
-  const CloNet<2>* net;     // parameters (kernel parameter space)
+  const CloFull* net;       // parameters (kernel parameter space)
   uint8_t* sA;              // two A tiles: 128 rows x 32 bf16 each, canonical K-major layout
   uint32_t sA_addr, sB_addr, mbar_addr;  // shared-window addresses
   uint32_t sB1_addr;        // W1 tile (first layer on the tensor cores)
@@ -63,7 +66,6 @@ template <> struct CloNet<3> {
   uint32_t wait_limit;      // polls per MMA wait before the CTA gives up
   bool row_ok;              // this thread's row exists (y < ny)
   uint32_t phase;           // mbarrier phase of this evaluation (alternates per use)
-  __device__ __forceinline__ float operator[](int k) const { return net->v[k]; }
 };
 constexpr int CLO_TILE_A_BYTES = 128 * 64;
 // First layer (9 -> 32) on the tensor cores as well: one K = 16 MMA of the
@@ -199,7 +201,7 @@ __device__ __forceinline__ float closure_warp(const CloNet<2>& w, const float (&
     // k = 10 s + j: part s (high, middle, low) of feature j, 30 and 31 zero
     float x[CLO_IN + 1];
 #pragma unroll
-    for (int j = 0; j < CLO_IN; ++j) x[j] = __fmul_rn(__fsub_rn(xr[j], w.v[CLO_MEAN + j]), w.v[CLO_ISCALE + j]);
+    for (int j = 0; j < CLO_IN; ++j) x[j] = __fmul_rn(__fsub_rn(xr[j], w.mean[j]), w.iscale[j]);
     x[CLO_IN] = 0.0f;
     uint32_t k[16];
 #pragma unroll
@@ -287,7 +289,7 @@ __device__ __forceinline__ float closure_warp(const CloNet<2>& w, const float (&
   const float a = __shfl_sync(0xffffffffu, z0[0], src), b = __shfl_sync(0xffffffffu, z1[0], src);
   const float c = __shfl_sync(0xffffffffu, z0[1], src), d = __shfl_sync(0xffffffffu, z1[1], src);
   const float z = (lane & 16) ? ((lane & 8) ? d : c) : ((lane & 8) ? b : a);
-  return Ops1::softplus(__fadd_rn(z, w.v[CLO_B3]));
+  return Ops1::softplus(__fadd_rn(z, w.b3));
 }
 __device__ __forceinline__ float closure_step_r(const CloNet<2>& w, const float (&x)[CLO_IN]) {
   return closure_warp(w, x);
@@ -375,7 +377,7 @@ __device__ __forceinline__ void clo_give_up(const CloNet<3>& c) {
 // mbarrier completes twice per evaluation (parities 0 and 1), else once (the
 // evaluation's parity).
 __device__ __forceinline__ float closure_mlp_tc(const CloNet<3>& c, const float (&xr)[CLO_IN]) {
-  const CloNet<2>& w = *c.net;
+  const CloFull& w = *c.net;
   const int r = threadIdx.y * 32 + threadIdx.x;
   float x[CLO_IN];
 #pragma unroll

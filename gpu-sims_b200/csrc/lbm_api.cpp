@@ -127,8 +127,7 @@ void free_all(Ctx* c) {
   for (auto& g : c->graph)
     if (g) cudaGraphExecDestroy(g);
   void* ptrs[] = {c->fbuf[0], c->fbuf[1], c->pop,      c->mask,     c->flags, c->links,
-                  c->rho,     c->u,       c->status,   c->partials, c->sums,  c->staging,
-                  c->clo_frag};
+                  c->rho,     c->u,       c->status,   c->partials, c->sums,  c->staging};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (c->own_stream) cudaStreamDestroy(c->own_stream);
@@ -289,8 +288,9 @@ int lbm_create(const lbm_desc* desc, lbm_ctx** out) {
       (rc = dev_alloc(c, &c->u, 3 * n, "cudaMalloc(u)")) ||
       (rc = dev_alloc(c, &c->status, 4, "cudaMalloc(status)")) ||
       (rc = dev_alloc(c, &c->partials, 4 * (size_t)c->nblk_cons, "cudaMalloc(partials)")) ||
-      (rc = dev_alloc(c, &c->sums, 4, "cudaMalloc(sums)")))
+      (rc = dev_alloc(c, &c->sums, 4 + (c->pop ? lbm::CLO_FRAG_WORDS / 2 : 0), "cudaMalloc(sums)")))
     return bail(rc);
+  if (c->pop) c->clo_frag = c->sums + 4;  // behind the sums: lbm_set_closure allocates nothing
 
   cudaStream_t s = c->stream;
   if (c->fbuf[0]) {
@@ -362,11 +362,6 @@ int lbm_set_closure(lbm_ctx* c, const float* net) {
     for (int k = 0; k < LBM_CLOSURE_FLOATS; ++k)
       if (!std::isfinite(net[k])) return fail(c, LBM_ERR_INVALID_ARG, "closure network has a non-finite value");
   }
-  if (net && !c->clo_frag) {
-    uint32_t* p = nullptr;
-    if (int rc = dev_alloc(c, &p, lbm::CLO_FRAG_WORDS, "cudaMalloc(closure)")) return rc;
-    c->clo_frag = p;
-  }
   // Captured step graphs hold the old network by value: rebuild them.
   CK(cudaStreamSynchronize(c->stream), "set_closure sync");
   drop_graphs(c);
@@ -377,8 +372,8 @@ int lbm_set_closure(lbm_ctx* c, const float* net) {
   if (net) {
     uint32_t words[lbm::CLO_FRAG_WORDS];
     lbm::clo_fragments(c->clo, words);
+    // from pageable memory: staged before the call returns, and in order with the steps
     CK(cudaMemcpyAsync(c->clo_frag, words, sizeof(words), cudaMemcpyHostToDevice, c->stream), "upload closure");
-    CK(cudaStreamSynchronize(c->stream), "upload closure sync");
   }
   return c->initialized ? prepare_graphs(c) : LBM_OK;
 }

@@ -188,7 +188,7 @@ struct Ctx {
   // value; weights already rounded to bf16
   bool closure = false;
   float clo[LBM_CLOSURE_FLOATS] = {};
-  void* clo_frag = nullptr;   // device: its layers as matrix fragments (clo_fragments)
+  void* clo_frag = nullptr;   // device, in the allocation of sums: its layers as matrix fragments (clo_fragments)
   uint32_t clo_wait_polls = LBM_CLO_WAIT_LIMIT;  // polls per tensor-core MMA wait
   // blocks of a row-tile step, 0: the whole chip's (a batch runs several domains
   // side by side)

@@ -184,7 +184,7 @@ __global__ void __launch_bounds__(STEP_THREADS, LBM_TC_MINB)
     k_phys_step_tc(PhysParams p, void* __restrict__ pop_v, const uint8_t* __restrict__ flags,
                    const uint32_t* __restrict__ links, float* __restrict__ rho_o,
                    float* __restrict__ u_o, unsigned* __restrict__ status,
-                   const __grid_constant__ CloNet<2> net, uint32_t wait_polls) {
+                   const __grid_constant__ CloFull net, uint32_t wait_polls) {
   static_assert(STEP_THREADS == 128, "one MMA row per thread");
   __shared__ __align__(1024) uint8_t sA[2 * CLO_TILE_A_BYTES];
   __shared__ __align__(1024) uint8_t sB[CLO_HID * 64];
@@ -271,7 +271,11 @@ __global__ void __launch_bounds__(STEP_THREADS, LBM_TC_MINB)
 template <int SGS> CloNet<SGS> net_of(const Ctx&) { return CloNet<SGS>{}; }
 template <> CloNet<2> net_of<2>(const Ctx& c) {
   CloNet<2> n;
-  for (int k = 0; k < CLO_FLOATS; ++k) n.v[k] = c.clo[k];
+  for (int k = 0; k < CLO_IN; ++k) {
+    n.mean[k] = c.clo[CLO_MEAN + k];
+    n.iscale[k] = c.clo[CLO_ISCALE + k];
+  }
+  n.b3 = c.clo[CLO_B3];
   n.frag = static_cast<const uint4*>(c.clo_frag);
   return n;
 }
@@ -373,7 +377,8 @@ cudaError_t dispatch_force(const Ctx& c, int P, bool wm, cudaStream_t s) {
 template <int PREC, int COLL>
 cudaError_t launch_step_tc(const Ctx& c, int P, bool wm, cudaStream_t s) {
   const PhysGeom& G = c.pp.g;
-  const CloNet<2> net = net_of<2>(c);
+  CloFull net;
+  for (int k = 0; k < CLO_FLOATS; ++k) net.v[k] = c.clo[k];
   const dim3 blk(32, STEP_BY, 1);
   const dim3 grd((G.nx + 31) / 32, (G.ny + STEP_BY - 1) / STEP_BY, (G.nz + LBM_TC_ZPB - 1) / LBM_TC_ZPB);
 #define LBM_STEP_LAUNCH(WM, PAR)                                          \
