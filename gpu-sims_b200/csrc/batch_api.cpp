@@ -38,13 +38,17 @@ struct lbm_batch {
   uint32_t ntiles = 0;
   int grid = 0;
   cudaStream_t own = nullptr, stream = nullptr;
-  cudaGraphExec_t graph[2] = {nullptr, nullptr};
+  cudaGraphExec_t graph[2] = {nullptr, nullptr};       // of the schedule
+  cudaGraphExec_t lane_graph[2] = {nullptr, nullptr};  // of the lanes
   static constexpr int kGraphSteps = 16;
   // graph mode's lanes (plan_lanes): each a list of domains, run one after the
   // other, the lanes side by side on lane_blocks blocks each; empty: one tile
   // launch a step
   std::vector<std::vector<int>> lanes;
   int lane_blocks = 0;
+  bool use_lanes = true;        // false when lbm_batch_autotune measured the tile kernel faster
+  int64_t lane_payoff = 0;      // steps that pay for building a lanes graph
+  int64_t lane_waited = 0;      // steps graph mode took without lanes meanwhile
   std::vector<cudaStream_t> lane_streams;  // for the capture
   std::vector<cudaEvent_t> lane_events;
   int parity = 0;
@@ -85,12 +89,22 @@ int balloc(lbm_batch* b, void** p, size_t bytes, const char* what) {
   return LBM_OK;
 }
 
-void drop_graphs(lbm_batch* b) {
-  for (auto& g : b->graph)
+void drop_graphs(cudaGraphExec_t (&graphs)[2]) {
+  for (auto& g : graphs)
     if (g) {
       cudaGraphExecDestroy(g);
       g = nullptr;
     }
+}
+
+// Whether graph mode runs lanes.  The schedule's tile shape is not theirs, so
+// their graphs outlive a change of it.
+bool lanes_on(const lbm_batch* b) { return !b->sched.persistent && b->use_lanes && !b->lanes.empty(); }
+
+// Whether the next graph of a call with `left` steps to go is the lanes' (plan_lanes).
+bool lanes_next(const lbm_batch* b, int64_t left) {
+  return lanes_on(b) && left > lbm_batch::kGraphSteps &&
+         (b->lane_graph[b->parity] || b->lane_waited + left >= b->lane_payoff);
 }
 
 lbm::BatchLaunch launch_of(const lbm_batch* b) {
@@ -155,7 +169,7 @@ int build_tiles(lbm_batch* b) {
                       cudaMemcpyHostToDevice, b->stream),
       "upload tile table");
   BCK(cudaStreamSynchronize(b->stream), "tile table sync");
-  drop_graphs(b);
+  drop_graphs(b->graph);
   b->grid = 0;
   if (b->sched.persistent) BCK(lbm::batch_persistent_grid(launch_of(b), &b->grid), "persistent grid");
   return LBM_OK;
@@ -202,6 +216,12 @@ bool valid_schedule(const lbm_batch_schedule& s) {
 // is no shorter than its own.  Estimates from B200: a round of tiles (one per
 // block) 2.2 us in 2-byte storage and 3.7 us in fp32, 4 us to start and end a
 // launch; the tile kernel 35.7 and 26.5 nodes/ns.
+//
+// A lanes graph has a node for every domain and step, and takes about 0.4 ms and
+// 4 us a node to build, where the tile kernel's takes 0.2 ms in all (32 domains
+// 2.3 ms, 128 domains 8 ms, 256 domains 16 ms).  lane_payoff is the number of
+// steps in which the lanes gain that; until a batch has that many before it,
+// in one call or several, it runs the tile kernel's graph.
 void plan_lanes(lbm_batch* b) {
   b->lanes.clear();
   const size_t nd = b->dom.size();
@@ -213,7 +233,8 @@ void plan_lanes(lbm_batch* b) {
   std::vector<int> order(nd);
   for (size_t i = 0; i < nd; ++i) order[i] = (int)i;
   std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return tiles[x] > tiles[y]; });
-  double best = 0.95 * (double)b->total_nodes / (f32 ? 26.5e3 : 35.7e3);  // us a step
+  const double tile_us = (double)b->total_nodes / (f32 ? 26.5e3 : 35.7e3);  // a step
+  double best = 0.95 * tile_us;
   for (int n : {2, 4, 8, 16}) {
     if ((size_t)n > nd) break;
     const int blocks = 296 / n;
@@ -229,6 +250,10 @@ void plan_lanes(lbm_batch* b) {
       best = t;
       b->lanes = std::move(lanes);
       b->lane_blocks = blocks;
+      // gained in a step: at least 0.3 of it (the estimates are near for large batches,
+      // where they part less than the times do for small ones)
+      b->lane_payoff =
+          (int64_t)((400.0 + 4.0 * lbm_batch::kGraphSteps * (double)nd) / std::max(tile_us - t, 0.3 * t));
     }
   }
 }
@@ -267,10 +292,10 @@ cudaError_t capture_lanes(lbm_batch* b, int slot) {
 // Captures kGraphSteps steps from parity `slot`, without the moment write:
 // the lanes' steps, kGraphSteps launches of the tile kernel, or in persistent mode one
 // cooperative launch that takes all of them with grid barriers between.
-int build_graph(lbm_batch* b, int slot) {
+int build_graph(lbm_batch* b, int slot, bool lanes) {
   const lbm::BatchLaunch L = launch_of(b);
   cudaGraph_t g = nullptr;
-  const bool lanes = !b->sched.persistent && !b->lanes.empty();
+  cudaGraphExec_t& graph = lanes ? b->lane_graph[slot] : b->graph[slot];
   while (lanes && b->lane_streams.size() + 1 < b->lanes.size()) {
     cudaStream_t s = nullptr;
     BCK(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking), "lane stream");
@@ -297,10 +322,10 @@ int build_graph(lbm_batch* b, int slot) {
     if (g) cudaGraphDestroy(g);
     return bcuda(b, e != cudaSuccess ? e : e2, "capture batch graph");
   }
-  e = cudaGraphInstantiate(&b->graph[slot], g, 0);
+  e = cudaGraphInstantiate(&graph, g, 0);
   cudaGraphDestroy(g);
   if (e != cudaSuccess) return bcuda(b, e, "instantiate batch graph");
-  BCK(cudaGraphUpload(b->graph[slot], b->stream), "upload batch graph");
+  BCK(cudaGraphUpload(graph, b->stream), "upload batch graph");
   return LBM_OK;
 }
 
@@ -313,9 +338,12 @@ int run_steps(lbm_batch* b, int nsteps) {
   int left = nsteps;
   while (left > lbm_batch::kGraphSteps) {
     const int slot = b->parity;
-    if (!b->graph[slot])
-      if (int rc = build_graph(b, slot)) return rc;
-    BCK(cudaGraphLaunch(b->graph[slot], b->stream), "batch graph launch");
+    const bool lanes = lanes_next(b, left);
+    const cudaGraphExec_t& graph = lanes ? b->lane_graph[slot] : b->graph[slot];
+    if (!graph)
+      if (int rc = build_graph(b, slot, lanes)) return rc;
+    BCK(cudaGraphLaunch(graph, b->stream), "batch graph launch");
+    if (!lanes) b->lane_waited += lbm_batch::kGraphSteps;
     left -= lbm_batch::kGraphSteps;
   }
   if (b->sched.persistent) {
@@ -331,14 +359,20 @@ int run_steps(lbm_batch* b, int nsteps) {
 }
 
 // Autotune results for this process, keyed by (precision, collision,
-// log2 of total nodes, log2 of domain count); optionally persisted as text
-// lines in $LBM_AUTOTUNE_CACHE.
+// log2 of total nodes, log2 of domain count, whether lanes are planned); optionally
+// persisted as text lines in $LBM_AUTOTUNE_CACHE.  A line starts with its version:
+// those without one were measured without lanes and are passed over.
+struct Tuned {
+  lbm_batch_schedule sched;
+  bool lanes;  // graph mode's lanes were the fastest
+};
+using TuneKey = std::tuple<int, int, int, int, int>;
 std::mutex g_tune_mu;
-std::map<std::tuple<int, int, int, int>, lbm_batch_schedule> g_tune;
+std::map<TuneKey, Tuned> g_tune;
 
-std::tuple<int, int, int, int> tune_key(const lbm_batch* b) {
+TuneKey tune_key(const lbm_batch* b) {
   return {b->precision, b->collision, (int)std::lround(std::log2((double)std::max<uint64_t>(b->total_nodes, 1))),
-          (int)std::lround(std::log2((double)std::max<size_t>(b->dom.size(), 1)))};
+          (int)std::lround(std::log2((double)std::max<size_t>(b->dom.size(), 1))), b->lanes.empty() ? 0 : 1};
 }
 
 void cache_load() {
@@ -346,25 +380,28 @@ void cache_load() {
   if (!path) return;
   FILE* f = std::fopen(path, "r");
   if (!f) return;
-  int p, c, n, d, r, z, pe;
-  while (std::fscanf(f, "%d %d %d %d %d %d %d", &p, &c, &n, &d, &r, &z, &pe) == 7) {
+  int p, c, n, d, l, r, z, pe, on;
+  char line[256];
+  while (std::fgets(line, sizeof(line), f)) {
+    if (std::sscanf(line, "v2 %d %d %d %d %d %d %d %d %d", &p, &c, &n, &d, &l, &r, &z, &pe, &on) != 9) continue;
     lbm_batch_schedule s{};
     s.struct_size = sizeof(s);
     s.rows_per_block = r;
     s.z_per_thread = z;
     s.persistent = pe;
     s.spin_limit_cycles = 2000000000LL;
-    if (valid_schedule(s)) g_tune[{p, c, n, d}] = s;
+    if (valid_schedule(s)) g_tune[{p, c, n, d, l}] = {s, on != 0};
   }
   std::fclose(f);
 }
 
-void cache_store(const std::tuple<int, int, int, int>& k, const lbm_batch_schedule& s) {
+void cache_store(const TuneKey& k, const Tuned& t) {
   const char* path = std::getenv("LBM_AUTOTUNE_CACHE");
   if (!path) return;
   if (FILE* f = std::fopen(path, "a")) {
-    std::fprintf(f, "%d %d %d %d %d %d %d\n", std::get<0>(k), std::get<1>(k), std::get<2>(k),
-                 std::get<3>(k), s.rows_per_block, s.z_per_thread, s.persistent);
+    std::fprintf(f, "v2 %d %d %d %d %d %d %d %d %d\n", std::get<0>(k), std::get<1>(k), std::get<2>(k),
+                 std::get<3>(k), std::get<4>(k), t.sched.rows_per_block, t.sched.z_per_thread, t.sched.persistent,
+                 t.lanes ? 1 : 0);
     std::fclose(f);
   }
 }
@@ -495,7 +532,8 @@ int lbm_batch_create(const lbm_desc* descs, int n, lbm_batch** out) {
 int lbm_batch_destroy(lbm_batch* b) {
   if (!b) return LBM_OK;
   if (b->stream) cudaStreamSynchronize(b->stream);
-  drop_graphs(b);
+  drop_graphs(b->graph);
+  drop_graphs(b->lane_graph);
   for (auto s : b->lane_streams) cudaStreamDestroy(s);
   for (auto v : b->lane_events) cudaEventDestroy(v);
   for (void* p : b->allocs) cudaFree(p);
@@ -622,14 +660,18 @@ int lbm_batch_read_populations(lbm_batch* b, int d, float* f, size_t n) {
   return LBM_OK;
 }
 
-int lbm_batch_set_schedule(lbm_batch* b, const lbm_batch_schedule* s) {
+// A schedule as it stands, and whether its graph mode may run lanes.
+static int apply_schedule(lbm_batch* b, const lbm_batch_schedule* s, bool lanes) {
   if (!b || !s) return bfail(b, LBM_ERR_INVALID_ARG, "NULL argument");
   if (s->struct_size != sizeof(lbm_batch_schedule) || !valid_schedule(*s))
     return bfail(b, LBM_ERR_INVALID_ARG, "schedule out of range (rows 1/2/4/8, z 1..16, persistent 0/1)");
   BCK(cudaStreamSynchronize(b->stream), "schedule sync");
   b->sched = *s;
+  b->use_lanes = lanes;
   return build_tiles(b);
 }
+
+int lbm_batch_set_schedule(lbm_batch* b, const lbm_batch_schedule* s) { return apply_schedule(b, s, true); }
 
 int lbm_batch_get_schedule(lbm_batch* b, lbm_batch_schedule* s) {
   if (!b || !s) return bfail(b, LBM_ERR_INVALID_ARG, "NULL argument");
@@ -652,9 +694,9 @@ int lbm_batch_autotune(lbm_batch* b, int trial_steps, lbm_batch_schedule* best_o
     }
     auto it = g_tune.find(key);
     if (it != g_tune.end()) {
-      lbm_batch_schedule s = it->second;
+      lbm_batch_schedule s = it->second.sched;
       s.spin_limit_cycles = b->sched.spin_limit_cycles;
-      if (int rc = lbm_batch_set_schedule(b, &s)) return rc;
+      if (int rc = apply_schedule(b, &s, it->second.lanes)) return rc;
       if (best_out) *best_out = b->sched;
       return LBM_OK;
     }
@@ -669,9 +711,19 @@ int lbm_batch_autotune(lbm_batch* b, int trial_steps, lbm_batch_schedule* best_o
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
-  lbm_batch_schedule best = b->sched;
-  float best_ms = 1e30f;
+  // the fastest of each mode (graph mode by the tile kernel, persistent mode)
+  lbm_batch_schedule best[2] = {b->sched, b->sched};
+  float best_ms[2] = {1e30f, 1e30f};  // a step
   int rc = LBM_OK;
+  auto timed = [&](int steps) {
+    cudaEventRecord(e0, b->stream);
+    rc = run_steps(b, steps);
+    cudaEventRecord(e1, b->stream);
+    cudaEventSynchronize(e1);
+    float ms = 0.f;
+    cudaEventElapsedTime(&ms, e0, e1);
+    return ms / (float)steps;
+  };
   for (int pers = 0; pers <= 1 && rc == LBM_OK; ++pers)
     for (int rows : {2, 4, 8})
       for (int zt : {1, 2, 4, 8, 16}) {
@@ -680,19 +732,31 @@ int lbm_batch_autotune(lbm_batch* b, int trial_steps, lbm_batch_schedule* best_o
         s.z_per_thread = zt;
         s.persistent = pers;
         s.test_missing_blocks = 0;
-        if ((rc = lbm_batch_set_schedule(b, &s))) break;
+        if ((rc = apply_schedule(b, &s, false))) break;
         if ((rc = run_steps(b, 2))) break;  // warm (and build graphs)
-        cudaEventRecord(e0, b->stream);
-        if ((rc = run_steps(b, trial_steps))) break;
-        cudaEventRecord(e1, b->stream);
-        cudaEventSynchronize(e1);
-        float ms = 0.f;
-        cudaEventElapsedTime(&ms, e0, e1);
-        if (ms < best_ms) {
-          best_ms = ms;
-          best = s;
+        const float ms = timed(trial_steps);
+        if (rc) break;
+        if (ms < best_ms[pers]) {
+          best_ms[pers] = ms;
+          best[pers] = s;
         }
       }
+  // The lanes run whole graphs, whatever the trial's length: one to warm and one
+  // timed, over the same steps a call of theirs takes.
+  bool lanes = false;
+  if (rc == LBM_OK && !b->lanes.empty() && (rc = apply_schedule(b, &best[0], true)) == LBM_OK) {
+    b->lane_waited = b->lane_payoff;
+    if (!b->lane_graph[b->parity]) rc = build_graph(b, b->parity, true);
+    float ms = 1e30f;
+    for (int i = 0; i < 2 && rc == LBM_OK; ++i) {
+      cudaEventRecord(e0, b->stream);
+      if (cudaError_t e = cudaGraphLaunch(b->lane_graph[b->parity], b->stream)) rc = bcuda(b, e, "batch graph launch");
+      cudaEventRecord(e1, b->stream);
+      cudaEventSynchronize(e1);
+      cudaEventElapsedTime(&ms, e0, e1);
+    }
+    lanes = rc == LBM_OK && ms / lbm_batch::kGraphSteps < std::min(best_ms[0], best_ms[1]);
+  }
   cudaMemcpyAsync(pool, snap, b->pop_bytes, cudaMemcpyDeviceToDevice, b->stream);
   cudaStreamSynchronize(b->stream);
   cudaFree(snap);
@@ -700,14 +764,18 @@ int lbm_batch_autotune(lbm_batch* b, int trial_steps, lbm_batch_schedule* best_o
   cudaEventDestroy(e1);
   b->parity = parity0;
   for (auto& v : b->dom) v.parity = parity0;
-  if (rc) return rc;
-  if (int r2 = lbm_batch_set_schedule(b, &best)) return r2;
+  if (rc) {
+    b->use_lanes = true;
+    return rc;
+  }
+  const Tuned t{best[!lanes && best_ms[1] < best_ms[0]], lanes};
+  if (int r2 = apply_schedule(b, &t.sched, t.lanes)) return r2;
   {
     std::lock_guard<std::mutex> lock(g_tune_mu);
-    g_tune[key] = best;
-    cache_store(key, best);
+    g_tune[key] = t;
+    cache_store(key, t);
   }
-  if (best_out) *best_out = best;
+  if (best_out) *best_out = t.sched;
   return LBM_OK;
 }
 
@@ -727,14 +795,14 @@ int lbm_batch_get_info(lbm_batch* b, lbm_batch_info* info) {
 int lbm_batch_set_row_wait_limit(lbm_batch* b, int32_t polls) {
   if (!b) return bfail(nullptr, LBM_ERR_INVALID_ARG, "batch is NULL");
   BCK(cudaStreamSynchronize(b->stream), "set_row_wait_limit sync");
-  drop_graphs(b);
+  drop_graphs(b->lane_graph);
   for (auto& v : b->dom) v.row_wait_polls = polls < 0 ? (uint32_t)LBM_ROW_WAIT_LIMIT : (uint32_t)polls;
   return LBM_OK;
 }
 
-int lbm_batch_lanes(lbm_batch* b) {
+int lbm_batch_lanes(lbm_batch* b, int nsteps) {
   if (!b) return bfail(nullptr, LBM_ERR_INVALID_ARG, "batch is NULL");
-  return b->sched.persistent ? 0 : (int)b->lanes.size();
+  return lanes_next(b, nsteps) ? (int)b->lanes.size() : 0;
 }
 
 const char* lbm_batch_last_error(lbm_batch* b) { return b ? b->err.c_str() : lbm_last_error(nullptr); }

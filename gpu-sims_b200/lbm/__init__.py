@@ -223,7 +223,7 @@ _SIGS = {
     "lbm_jitter_lut": (C.c_int, [_P]),
     "lbm_step_streams_rows": (C.c_int, [_P]),
     "lbm_set_row_wait_limit": (C.c_int, [_P, C.c_int32]),
-    "lbm_batch_lanes": (C.c_int, [_P]),
+    "lbm_batch_lanes": (C.c_int, [_P, C.c_int]),
     "lbm_batch_set_row_wait_limit": (C.c_int, [_P, C.c_int32]),
     "lbm_set_closure": (C.c_int, [_P, _P]),
     "lbm_set_closure_wait_limit": (C.c_int, [_P, C.c_int32]),
@@ -612,9 +612,9 @@ class Batch:
         self._c(load().lbm_batch_autotune(self._h, trial_steps, C.byref(s)))
         return s
 
-    def lanes(self) -> int:
-        """Parallel lanes that graph mode runs (lbm_batch_lanes)."""
-        return load().lbm_batch_lanes(self._h)
+    def lanes(self, nsteps: int) -> int:
+        """Parallel lanes that step(nsteps) would start with (lbm_batch_lanes)."""
+        return load().lbm_batch_lanes(self._h, int(nsteps))
 
     def set_row_wait_limit(self, polls: int) -> None:
         """Testing hook, as Lattice.set_row_wait_limit for every domain."""

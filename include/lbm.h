@@ -470,9 +470,11 @@ typedef struct lbm_batch lbm_batch;
 
 typedef struct lbm_batch_schedule {
     uint32_t struct_size;
+    /* the tile kernel's shape, in either mode; lanes (lbm_batch_lanes) have none */
     int32_t  rows_per_block;      /* 1, 2, 4, 8: a block is 32 x rows threads */
     int32_t  z_per_thread;        /* 1..16 nodes along z per thread           */
-    int32_t  persistent;          /* 1 = one cooperative launch per call      */
+    int32_t  persistent;          /* 1 = one cooperative launch per call, 0 =
+                                     graphs: lanes or the tile kernel         */
     int64_t  spin_limit_cycles;   /* bound of a grid-barrier wait (persistent)*/
     int32_t  test_missing_blocks; /* testing only: barrier waits for this many
                                      blocks that never arrive -> TIMEOUT      */
@@ -482,7 +484,7 @@ typedef struct lbm_batch_info {
     uint32_t struct_size;
     int32_t  domains;
     uint64_t total_nodes;
-    uint32_t tiles;
+    uint32_t tiles;               /* of the tile kernel                       */
     int32_t  grid;                /* persistent grid size (0 in graph mode)   */
     uint64_t iteration;
     uint64_t device_bytes;
@@ -509,15 +511,20 @@ LBM_API int lbm_batch_read_moments(lbm_batch* b, int domain, float* rho, void* u
 LBM_API int lbm_batch_read_populations(lbm_batch* b, int domain, float* f, size_t n);
 LBM_API int lbm_batch_set_schedule(lbm_batch* b, const lbm_batch_schedule* s);
 LBM_API int lbm_batch_get_schedule(lbm_batch* b, lbm_batch_schedule* s);
-/* Times every schedule (rows 2/4/8 x z 1/2/4 x graph/persistent) for
- * trial_steps steps, keeps the fastest and restores the populations.  Results
- * are cached per (precision, collision, size class) for the process and, if
- * $LBM_AUTOTUNE_CACHE names a file, across processes. */
+/* Times every schedule (rows 2/4/8 x z 1/2/4/8/16 x graph/persistent) for
+ * trial_steps steps and, where lanes are planned, a graph of theirs (16 steps);
+ * keeps the fastest and restores the populations.  With lanes the schedule is
+ * that of the steps they leave over.  Results are cached per (precision,
+ * collision, size class, whether lanes are planned) for the process and, if
+ * $LBM_AUTOTUNE_CACHE names a file, across processes (lines of earlier library
+ * versions, measured without lanes, are passed over). */
 LBM_API int lbm_batch_autotune(lbm_batch* b, int trial_steps, lbm_batch_schedule* best);
-/* The parallel lanes that graph mode runs (16 steps of whole domains side by
- * side), 0 when it launches the tile kernel or the batch is in persistent mode;
- * < 0 on error. */
-LBM_API int lbm_batch_lanes(lbm_batch* b);
+/* The parallel lanes that an lbm_batch_step of nsteps steps would start with now
+ * (16 steps of whole domains side by side), 0 when it would launch the schedule's
+ * kernel: in persistent mode, where that is estimated or measured faster, for
+ * calls of 16 steps and fewer, and until the steps asked for pay for building the
+ * lanes' graph (some tens to hundreds).  < 0 on error. */
+LBM_API int lbm_batch_lanes(lbm_batch* b, int nsteps);
 /* lbm_set_row_wait_limit of every domain, for the lanes' steps. */
 LBM_API int lbm_batch_set_row_wait_limit(lbm_batch* b, int32_t polls);
 LBM_API int lbm_batch_get_info(lbm_batch* b, lbm_batch_info* info);

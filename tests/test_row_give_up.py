@@ -65,13 +65,13 @@ def test_lanes_give_up_and_recover(gpu):
     shape = (96, 80, 40)
     descs = [gpu.default_desc(nx=shape[0], ny=shape[1], nz=shape[2], mode=gpu.MODE_PHYSICS, precision=1, tau=0.6)] * 16
     b = gpu.Batch(descs)
-    assert b.lanes() > 0
     got = []
     for limit in (-1, 0, -1):
         for i in range(len(descs)):
             b.init_from_moments(i, *moments(shape, i))
         b.set_row_wait_limit(limit)
-        b.step(32)  # graphs of lanes; the last sixteen steps are the tile kernel's
+        assert b.lanes(400) > 0
+        b.step(400)  # graphs of lanes; the last sixteen steps are the tile kernel's
         if limit == 0:
             with pytest.raises(gpu.LbmError) as e:
                 b.sync()
