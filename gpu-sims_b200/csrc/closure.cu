@@ -64,7 +64,8 @@ namespace {
 // Box filter: one thread per coarse node, Favre averages of factor^3 fine
 // nodes accumulated in fp64.  Consecutive threads take consecutive coarse x,
 // so a warp reads contiguous fine rows: V values a load where the factor allows
-// (single values keep the load units busy: k_box_filter_any), and for F = 2 or 4 a
+// (single values keep the load units busy: k_box_filter_any, written out because
+// the template below with V = 1 takes 117 us for 288^3 / 9 where this takes 104), and for F = 2 or 4 a
 // plane's rows in flight together.  Bound by HBM at factor 4: 512^3 331 us = 6.5
 // TB/s (351 with single loads), 256^3 47.6 us (52.2), factor 2 61.6 (88), factor 8
 // 74 (90).

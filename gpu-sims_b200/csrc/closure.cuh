@@ -155,7 +155,9 @@ __device__ __forceinline__ typename O::F closure_mlp(const W& w, const typename 
 // products (mma.sync m16n8k16, bf16 in, fp32 accumulators), 32 nodes a warp at a
 // time.  The weights are bf16 values already; every activation enters as the sum
 // of three bf16 numbers (8 + 8 + 8 bits, the whole fp32 significand), so each
-// product is exact and only the fp32 sums round, as on the CUDA cores.
+// product is exact and only sums round: those of the matrix unit's fp32
+// accumulation, whose order and rounding are its own and not those of a chain of
+// fused multiply-adds (the step's error against 64 bits, below, is the same).
 //
 // Why not tcgen05 here: the layers are 9 x 32 and 32 x 32, so a node's chain is
 // features -> layer -> layer -> r, and the block-wide round trips through shared

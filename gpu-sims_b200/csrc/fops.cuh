@@ -50,9 +50,6 @@ struct Ops2 {
   static __device__ __forceinline__ F sqrt(F a) { return make_float2(__fsqrt_rn(a.x), __fsqrt_rn(a.y)); }
   static __device__ __forceinline__ F log(F a) { return make_float2(Ops1::log(a.x), Ops1::log(a.y)); }
   static __device__ __forceinline__ F relu(F a) { return make_float2(fmaxf(a.x, 0.0f), fmaxf(a.y, 0.0f)); }
-  static __device__ __forceinline__ F softplus(F z) {
-    return make_float2(Ops1::softplus(z.x), Ops1::softplus(z.y));
-  }
 };
 }  // namespace
 }  // namespace lbm

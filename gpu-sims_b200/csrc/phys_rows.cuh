@@ -5,10 +5,11 @@
 // A tile is R consecutive rows of one z-plane.  In each of the 19 slot arrays
 // its values are one contiguous run of R * px elements, fetched by one
 // cp.async.bulk and written back by one (two where a row at a y face comes
-// from another place).  One producer warp issues them and resolves everything that depends on the row only: the parity, the periodic
-// wraps, and the half-way bounce-back of the y and z faces (the same location
-// of the pair's other slot array).  The x faces' bounce-back values (one
-// element per row and array) arrive by 4-byte cp.async next to the rows.
+// from another place).  Four service warps issue them and resolve everything
+// that depends on the row only: the parity, the periodic wraps, and the half-way
+// bounce-back of the y and z faces (the same location of the pair's other slot
+// array).  The x faces' bounce-back values (one element per row and array) arrive
+// by 4-byte cp.async next to the rows.
 // Consumer threads own two x-adjacent nodes for the whole launch; every access
 // is a fixed offset from a few per-thread bases, the slots at x+1 of the
 // c_x = +1 pairs included.
@@ -317,21 +318,17 @@ __device__ __noinline__ void rows_land(uint32_t full, const volatile uint32_t* c
 constexpr int ROWS_NA = (Q + ROWS_SERV - 1) / ROWS_SERV;  // arrays of a service warp: part, part + ROWS_SERV, ...
 constexpr uint64_t ROWS_MOST_BYTES = 1ull << 36;          // of a store (32-bit offsets of 16 bytes, below)
 
-// The tiles of one domain in a block's walk: `count` of them from tile `first`
-// on, `stride` apart.
-struct RowSeg {
+// A block's walk: `count` tiles from tile `first` on, `stride` apart.
+struct RowRun {
   RowTiles rt;
   uint32_t first, stride, count;
 };
 
-// A service warp's part of a segment: loads ahead of the collision and writes
-// back behind it.  One lane issues the copies of the warp's arrays: their
-// operands are then uniform over the warp, and each costs a handful of
-// instructions.  The segment's rows have left the stages when it ends, so the
-// next one (another domain) starts from empty stages.  False when a wait gave
-// up.
+// A service warp's part of a block: loads ahead of the collision and writes back
+// behind it.  One lane issues the copies of the warp's arrays: their operands are
+// then uniform over the warp, and each costs a handful of instructions.
 template <int PREC>
-__device__ __forceinline__ bool rows_service(const PhysGeom& G, const RowSeg& sg, void* pop, int P, int part,
+__device__ __forceinline__ void rows_service(const PhysGeom& G, const RowRun& run, void* pop, int P, int part,
                                              uint32_t stage0, const RowBars& B, uint32_t stages, RowStage& st_) {
   using T = typename Store<PREC>::T;
   constexpr uint32_t EB = sizeof(T);
@@ -354,10 +351,10 @@ __device__ __forceinline__ bool rows_service(const PhysGeom& G, const RowSeg& sg
   uint32_t side_dst;
   const ptrdiff_t side_src = side_offset<PREC>(G, P, side_e, side_dst) * (ptrdiff_t)EB;
   RowWalk wl, ws;  // of the loads and of the stores
-  wl.start(sg.first, sg.stride, sg.rt.tiles_y);
+  wl.start(run.first, run.stride, run.rt.tiles_y);
   ws = wl;
   auto load = [&](uint32_t s) {
-    const int z = wl.z, y0 = wl.ty * sg.rt.R, rows = min(sg.rt.R, G.ny - y0);
+    const int z = wl.z, y0 = wl.ty * run.rt.R, rows = min(run.rt.R, G.ny - y0);
     const uint32_t st = stage0 + s * rows_stage<PREC>(), bar = B.full + 8 * s;
     const char* at = base + lin(G, 0, y0, z) * EB;
     const bool in = inner_tile(G, y0, z, rows);
@@ -390,25 +387,25 @@ __device__ __forceinline__ bool rows_service(const PhysGeom& G, const RowSeg& sg
       }
     }
     asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
-    wl.next(sg.rt.tiles_y);
+    wl.next(run.rt.tiles_y);
   };
   uint32_t loaded = 0, sl = st_.s;
 #pragma unroll 1
-  for (; loaded < min(stages, sg.count); ++loaded) {
+  for (; loaded < min(stages, run.count); ++loaded) {
     load(sl);
     if (++sl == stages) sl = 0;
   }
   uint32_t prev = 0;
   bool ok = true;
 #pragma unroll 1
-  for (uint32_t j = 0; j < sg.count; ++j) {
+  for (uint32_t j = 0; j < run.count; ++j) {
     ok = __all_sync(FULL, mbar_wait(B.done + 8 * st_.s, st_.ph, B.abort, ROWS_WAIT_LIMIT));
     if (!ok) {
       B.give_up();
       break;
     }
     if (lane == 0) {
-      const int z = ws.z, y0 = ws.ty * sg.rt.R, rows = min(sg.rt.R, G.ny - y0);
+      const int z = ws.z, y0 = ws.ty * run.rt.R, rows = min(run.rt.R, G.ny - y0);
       const uint32_t st = stage0 + st_.s * rows_stage<PREC>();
       char* at = base + lin(G, 0, y0, z) * EB;
       if (inner_tile(G, y0, z, rows)) {
@@ -432,9 +429,9 @@ __device__ __forceinline__ bool rows_service(const PhysGeom& G, const RowSeg& sg
       else asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
     }
     __syncwarp();
-    ws.next(sg.rt.tiles_y);
+    ws.next(run.rt.tiles_y);
     if (stages <= 2) prev = st_.s;
-    if ((j > 0 || stages <= 2) && loaded < sg.count) {
+    if ((j > 0 || stages <= 2) && loaded < run.count) {
       load(prev);
       ++loaded;
     }
@@ -449,12 +446,9 @@ __device__ __forceinline__ bool rows_service(const PhysGeom& G, const RowSeg& sg
                "barrier.cta.red.or.pred P2, 1, %2, P1;\n\tselp.b32 %0, 1, 0, P2;\n\t}\n"
                : "=r"(any) : "r"(ok ? 0u : 1u), "n"(32 * ROWS_SERV) : "memory");
   if (any) rows_land(B.full, B.loaded, loaded, stages);
-  return !any;
 }
 
-// One pair of nodes' step on a landed tile: stream from, and collide into, the
-// stage at st.
-// (cp holds what the collision reads, p everything.)
+// Where a consumer thread's two nodes lie in a stage.
 struct RowPair {
   int row, x;              // row within the tile, x of node A
   bool active;             // the thread has a pair
@@ -489,8 +483,10 @@ __host__ __device__ __forceinline__ RowPair row_pair(const PhysGeom& G, int R, i
   return q;
 }
 
+// One pair of nodes' step on a landed tile: stream from, and collide into, the
+// stage at st.
 template <int PREC, int COLL, int SGS, bool FORCE, bool WRITE_MOMENTS, bool OPEN>
-__device__ __forceinline__ void row_pair_step(const PhysParams& p, const PhysParams& cp, const PhysGeom& G, int moving,
+__device__ __forceinline__ void row_pair_step(const PhysParams& p, const PhysGeom& G,
                                               uint8_t* __restrict__ st, const RowPair& q,
                                               void* __restrict__ pop_v, const uint32_t* __restrict__ links,
                                               float* __restrict__ rho_o, float* __restrict__ u_o,
@@ -522,7 +518,7 @@ __device__ __forceinline__ void row_pair_step(const PhysParams& p, const PhysPar
   const uint32_t nid = (uint32_t)x + (uint32_t)G.nx * ((uint32_t)y + (uint32_t)G.ny * (uint32_t)z);
   const uint32_t flA = fl2 & 0xffu, flB = fl2 >> 8;
   const bool fluidA = !(flA & FLAG_SOLID), fluidB = !(flB & FLAG_SOLID);
-  if (moving && near_moving(moving, G, x, x + 1 < G.nx ? x + 1 : x, y, z)) {
+  if (p.any_moving_wall && near_moving(p, x, x + 1 < G.nx ? x + 1 : x, y, z)) {
     auto faces = [&](int xx, auto sel) {
       constexpr bool B = decltype(sel)::value != 0;
       const bool xlo = !G.per[0] && xx == 0, xhi = !G.per[0] && xx == G.nx - 1;
@@ -581,7 +577,7 @@ __device__ __forceinline__ void row_pair_step(const PhysParams& p, const PhysPar
   }
 
   float2 r2, ux2, uy2, uz2;
-  collide_t<Ops2, COLL, SGS, FORCE, PREC>(cp, CloNet<SGS>{}, g, r2, ux2, uy2, uz2);
+  collide_t<Ops2, COLL, SGS, FORCE, PREC>(p, CloNet<SGS>{}, g, r2, ux2, uy2, uz2);
 
   if (WRITE_MOMENTS && q.active && y < G.ny) {
     const uint32_t N = (uint32_t)G.n;
@@ -652,58 +648,56 @@ __device__ __forceinline__ uint32_t row_flags(const PhysGeom& G, const uint8_t* 
   return flags[nid] | b << 8;
 }
 
-// What a block needs of the domain whose tiles it walks.
-struct RowDomain {
+// A lattice's arrays.
+struct RowArrays {
   void* pop;
   const uint8_t* flags;
   const uint32_t* links;
   float *rho, *u;
 };
 
-// A consumer thread's part of a segment.  False when a wait gave up.
+// A consumer thread's part of a block.
 template <int PREC, int COLL, int SGS, bool FORCE, bool WRITE_MOMENTS, bool OPEN>
-__device__ __forceinline__ bool rows_consume(const PhysParams& p, const PhysParams& cp, const PhysGeom& G, int moving,
-                                             const RowSeg& sg, const RowDomain& D, uint8_t* sm, int tid, int P,
+__device__ __forceinline__ void rows_consume(const PhysParams& p, const PhysGeom& G,
+                                             const RowRun& run, const RowArrays& D, uint8_t* sm, int tid, int P,
                                              const RowBars& B, uint32_t polls, uint32_t stages, RowStage& st_) {
-  const RowPair q = row_pair<PREC>(G, sg.rt.R, sg.rt.tpr, tid);
+  const RowPair q = row_pair<PREC>(G, run.rt.R, run.rt.tpr, tid);
   RowWalk w;
-  w.start(sg.first, sg.stride, sg.rt.tiles_y);
-  int y = w.ty * sg.rt.R + q.row, z = w.z;
+  w.start(run.first, run.stride, run.rt.tiles_y);
+  int y = w.ty * run.rt.R + q.row, z = w.z;
   uint32_t fl = row_flags(G, D.flags, q, y, z);
   if (polls == 0) {  // testing: no wait at all, not even one that would end at once
     B.give_up();
-    return false;
+    return;
   }
-  for (uint32_t j = 0; j < sg.count; ++j) {
+  for (uint32_t j = 0; j < run.count; ++j) {
     const int yc = y, zc = z;
     const uint32_t flc = fl;
-    if (j + 1 < sg.count) {  // the next tile's flags, used one tile later
-      w.next(sg.rt.tiles_y);
-      y = w.ty * sg.rt.R + q.row;
+    if (j + 1 < run.count) {  // the next tile's flags, used one tile later
+      w.next(run.rt.tiles_y);
+      y = w.ty * run.rt.R + q.row;
       z = w.z;
       fl = row_flags(G, D.flags, q, y, z);
     }
     if (!__all_sync(FULL, mbar_wait(B.full + 8 * st_.s, st_.ph, B.abort, polls))) {
       B.give_up();
-      return false;
+      return;
     }
-    row_pair_step<PREC, COLL, SGS, FORCE, WRITE_MOMENTS, OPEN>(p, cp, G, moving, sm + st_.s * rows_stage<PREC>(), q,
+    row_pair_step<PREC, COLL, SGS, FORCE, WRITE_MOMENTS, OPEN>(p, G, sm + st_.s * rows_stage<PREC>(), q,
                                                                D.pop, D.links, D.rho, D.u, B.status, yc, zc, flc, P);
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncwarp();
     if ((threadIdx.x & 31) == 0) mbar_arrive(B.done + 8 * st_.s);
     st_.next(stages);
   }
-  return true;
 }
 
 // Set-up of a block: barriers, roles and the share of the registers; cons_warps
-// consumer warps take part.  SEGS is
-// called as segs(f) and calls f(p, cp, G, moving, segment, domain) for the
-// block's segments in order until f returns false.
-template <int PREC, int COLL, int SGS, bool FORCE, bool WRITE_MOMENTS, bool OPEN, class SEGS>
+// consumer warps take part.  with(f) calls f with the block's work; handed over
+// directly instead, 15 of the 32 kernels of a 2-byte format spilled, 428 bytes.
+template <int PREC, int COLL, int SGS, bool FORCE, bool WRITE_MOMENTS, bool OPEN, class WITH>
 __device__ __forceinline__ void rows_block(uint32_t stages, uint32_t cons_warps, uint32_t polls, unsigned* status, int P,
-                                           SEGS&& segs) {
+                                           WITH&& with) {
   extern __shared__ __align__(128) uint8_t sm[];
   __shared__ __align__(8) uint64_t bars[2 * ROWS_MAXST];
   __shared__ uint32_t s_abort, s_loaded[ROWS_SERV];
@@ -726,34 +720,33 @@ __device__ __forceinline__ void rows_block(uint32_t stages, uint32_t cons_warps,
   RowStage st;
   if (warp < ROWS_SERV) {
     if constexpr (rows_blocks<PREC, SGS>() > 1) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(ROWS_REGS_SERV));
-    segs([&](const PhysParams&, const PhysParams&, const PhysGeom& G, int, const RowSeg& sg, const RowDomain& D) {
-      return rows_service<PREC>(G, sg, D.pop, P, warp, smem_addr(sm), B, stages, st);
+    with([&](const PhysParams&, const PhysGeom& G, const RowRun& run, const RowArrays& D) {
+      rows_service<PREC>(G, run, D.pop, P, warp, smem_addr(sm), B, stages, st);
     });
     if ((threadIdx.x & 31) == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     return;
   }
   if constexpr (rows_blocks<PREC, SGS>() > 1) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(ROWS_REGS_CONS));
   if ((uint32_t)(warp - ROWS_SERV) >= cons_warps) return;
-  segs([&](const PhysParams& p, const PhysParams& cp, const PhysGeom& G, int moving, const RowSeg& sg,
-           const RowDomain& D) {
-    return rows_consume<PREC, COLL, SGS, FORCE, WRITE_MOMENTS, OPEN>(p, cp, G, moving, sg, D, sm,
-                                                                           (int)threadIdx.x - 32 * ROWS_SERV, P, B, polls, stages, st);
+  with([&](const PhysParams& p, const PhysGeom& G, const RowRun& run, const RowArrays& D) {
+    rows_consume<PREC, COLL, SGS, FORCE, WRITE_MOMENTS, OPEN>(p, G, run, D, sm, (int)threadIdx.x - 32 * ROWS_SERV, P, B,
+                                                              polls, stages, st);
   });
 }
 
-// One domain: block b takes tiles b, b + gridDim.x, ...
+// Block b takes tiles b, b + gridDim.x, ...
 template <int PREC, int COLL, int SGS, bool FORCE, bool WRITE_MOMENTS, bool OPEN>
 __global__ void __launch_bounds__(ROWS_THREADS, rows_blocks<PREC, SGS>())
     k_phys_rows(const __grid_constant__ PhysParams p, RowTiles rt, void* __restrict__ pop_v,
                 const uint8_t* __restrict__ flags, const uint32_t* __restrict__ links,
                 float* __restrict__ rho_o, float* __restrict__ u_o, unsigned* __restrict__ status, int P,
                 uint32_t polls) {
-  const RowDomain D{pop_v, flags, links, rho_o, u_o};
-  const RowSeg sg{rt, blockIdx.x, gridDim.x,
+  const RowArrays D{pop_v, flags, links, rho_o, u_o};
+  const RowRun run{rt, blockIdx.x, gridDim.x,
                   rt.ntiles <= blockIdx.x ? 0u : (rt.ntiles - blockIdx.x + gridDim.x - 1) / gridDim.x};
   const uint32_t cons_warps = (uint32_t)(rt.R * rt.tpr + 31) / 32;  // warps that have nodes
   rows_block<PREC, COLL, SGS, FORCE, WRITE_MOMENTS, OPEN>((uint32_t)rt.stages, cons_warps, polls, status, P, [&](auto&& f) {
-    if (sg.count) f(p, p, p.g, p.any_moving_wall, sg, D);
+    if (run.count) f(p, p.g, run, D);
   });
 }
 

@@ -359,16 +359,15 @@ __device__ __forceinline__ uint32_t offs(const PhysGeom& G, const Wrap& w) {
 // leaves through a moving face, so only nodes on such a face run the pass
 // (p.any_moving_wall holds bit f for each moving face f).  x_lo / x_hi are
 // the node group's first and last x.
-__device__ __forceinline__ bool near_moving(int m, const PhysGeom& G, int x_lo, int x_hi, int y, int z) {
+__device__ __forceinline__ bool near_moving(const PhysParams& p, int x_lo, int x_hi, int y, int z) {
+  const int m = p.any_moving_wall;
+  const PhysGeom& G = p.g;
   return ((m & (1 << LBM_FACE_XM)) && !G.per[0] && x_lo == 0) ||
          ((m & (1 << LBM_FACE_XP)) && !G.per[0] && x_hi == G.nx - 1) ||
          ((m & (1 << LBM_FACE_YM)) && !G.per[1] && y == 0) ||
          ((m & (1 << LBM_FACE_YP)) && !G.per[1] && y == G.ny - 1) ||
          ((m & (1 << LBM_FACE_ZM)) && !G.per[2] && z == 0) ||
          ((m & (1 << LBM_FACE_ZP)) && !G.per[2] && z == G.nz - 1);
-}
-__device__ __forceinline__ bool near_moving(const PhysParams& p, int x_lo, int x_hi, int y, int z) {
-  return near_moving(p.any_moving_wall, p.g, x_lo, x_hi, y, z);
 }
 
 // Index of pair pi among the five pairs with c_x = +1 (pairs 0, 3, 4, 5, 6).
