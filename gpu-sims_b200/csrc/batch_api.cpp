@@ -218,8 +218,9 @@ bool valid_schedule(const lbm_batch_schedule& s) {
 // launch; the tile kernel 35.7 and 26.5 nodes/ns.
 //
 // A lanes graph has a node for every domain and step, and takes about 0.4 ms and
-// 4 us a node to build, where the tile kernel's takes 0.2 ms in all (32 domains
-// 2.3 ms, 128 domains 8 ms, 256 domains 16 ms).  lane_payoff is the number of
+// 4 us a node to build, where the tile kernel's takes 0.14 ms in all (8 domains
+// 0.6 ms, 32 2.3, 128 9.5, 256 17; in a process's first batch 16 ms more, to load
+// the kernels).  lane_payoff is the number of
 // steps in which the lanes gain that; until a batch has that many before it,
 // in one call or several, it runs the tile kernel's graph.
 void plan_lanes(lbm_batch* b) {
@@ -769,6 +770,7 @@ int lbm_batch_autotune(lbm_batch* b, int trial_steps, lbm_batch_schedule* best_o
     return rc;
   }
   const Tuned t{best[!lanes && best_ms[1] < best_ms[0]], lanes};
+  if (!t.lanes) drop_graphs(b->lane_graph);
   if (int r2 = apply_schedule(b, &t.sched, t.lanes)) return r2;
   {
     std::lock_guard<std::mutex> lock(g_tune_mu);
