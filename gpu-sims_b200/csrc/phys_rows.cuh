@@ -750,8 +750,8 @@ __global__ void __launch_bounds__(ROWS_THREADS, rows_blocks<PREC, SGS>())
   });
 }
 
-// Tiles of a grid; R = 0 when a row does not fit or its copies would not start
-// on 16-byte boundaries.
+// Tiles of a grid; R = 0 when a row does not fit (more than 512 nodes, two a
+// consumer thread) or its copies would not start on 16-byte boundaries.
 inline RowTiles row_tiles(const PhysGeom& G) {
   RowTiles rt{};
   if (G.nx < 4 || G.px % 8 || G.px > ROWS_CAP || (uint64_t)Q * G.slot_stride * 4 >= ROWS_MOST_BYTES) return rt;
