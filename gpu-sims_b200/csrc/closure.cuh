@@ -169,6 +169,7 @@ __device__ __forceinline__ typename O::F closure_mlp(const W& w, const typename 
 // ---------------------------------------------------------------------------
 constexpr int CLO_ROW = 80;  // bytes of a node's row of features: 32 bf16 padded, so that
                              // eight rows of a matrix load hit distinct banks
+constexpr int CLO_WARPS = 4;  // warps of a block, at the most
 
 // fp32 values as sums of three bf16 numbers, two values a word.
 __device__ __forceinline__ void clo_split(float a, float b, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
@@ -195,7 +196,7 @@ __device__ __forceinline__ void clo_mma_sync(float (&c)[4], const uint32_t (&a)[
 // r of the warp's 32 nodes, lane = node, from their raw inputs.  Every lane of
 // the warp calls it.
 __device__ __forceinline__ float closure_warp(const CloNet<2>& w, const float (&xr)[CLO_IN]) {
-  __shared__ __align__(16) uint8_t rows[4][32 * CLO_ROW];  // blocks of up to four warps
+  __shared__ __align__(16) uint8_t rows[CLO_WARPS][32 * CLO_ROW];
   const int lane = threadIdx.x & 31, t = lane & 3;
   const int warp = (int)(threadIdx.y * blockDim.x + threadIdx.x) >> 5;
   const uint4* __restrict__ frag = w.frag;

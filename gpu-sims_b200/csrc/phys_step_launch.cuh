@@ -57,6 +57,7 @@ namespace {
 #ifndef LBM_STEP2_ROWS16
 #define LBM_STEP2_ROWS16 1
 #endif
+static_assert(STEP_BY <= CLO_WARPS, "closure_warp has rows for each warp of a block");
 template <int PREC, int SGS>
 constexpr int step2_rows() {
   return SGS == 2 ? STEP_BY : (PREC == LBM_PREC_F32 ? 1 : LBM_STEP2_ROWS16);
