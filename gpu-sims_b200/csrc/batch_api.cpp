@@ -477,7 +477,7 @@ int lbm_batch_create(const lbm_desc* descs, int n, lbm_batch** out) {
     b->total_nodes += v.n;
   }
   // periodic rows are padded for lanes where those are planned, and else, or
-  // where the padding does not fit, lie one behind the other
+  // where the batch does not fit with them padded, lie one behind the other
   auto layout = [&](bool rows) {
     pop_total = 0;
     for (int i = 0; i < n; ++i) {
@@ -493,13 +493,20 @@ int lbm_batch_create(const lbm_desc* descs, int n, lbm_batch** out) {
   const bool padded = layout(true) && !b->lanes.empty();
   if (!padded && !layout(false))
     return bail(bfail(b, LBM_ERR_UNSUPPORTED, "a domain exceeds 2^32 nodes per slot array"));
-  int pool_rc = balloc(b, &pop, pop_total, "cudaMalloc(population pool)");
-  if (pool_rc == LBM_ERR_OUT_OF_MEMORY && padded && layout(false))
-    pool_rc = balloc(b, &pop, pop_total, "cudaMalloc(population pool)");
-  if (pool_rc) return bail(pool_rc);
-  if (int rc = balloc(b, &aux, aux_total, "cudaMalloc(aux pool)")) return bail(rc);
-  if (int rc = balloc(b, &dd, n * sizeof(lbm::BatchDomain), "cudaMalloc(tile table)")) return bail(rc);
-  if (int rc = balloc(b, &st, 256, "cudaMalloc(status)")) return bail(rc);
+  auto arrays = [&]() -> int {
+    if (int rc = balloc(b, &pop, pop_total, "cudaMalloc(population pool)")) return rc;
+    if (int rc = balloc(b, &aux, aux_total, "cudaMalloc(aux pool)")) return rc;
+    if (int rc = balloc(b, &dd, n * sizeof(lbm::BatchDomain), "cudaMalloc(tile table)")) return rc;
+    return balloc(b, &st, 256, "cudaMalloc(status)");
+  };
+  int rc_arrays = arrays();
+  if (rc_arrays == LBM_ERR_OUT_OF_MEMORY && padded && layout(false)) {
+    for (void* p : b->allocs) cudaFree(p);
+    b->allocs.clear();
+    b->dev_bytes = 0;
+    rc_arrays = arrays();
+  }
+  if (rc_arrays) return bail(rc_arrays);
   b->pop_bytes = pop_total;
   b->d_dom = static_cast<lbm::BatchDomain*>(dd);
   b->status = static_cast<unsigned*>(st);

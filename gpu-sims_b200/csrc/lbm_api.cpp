@@ -123,13 +123,23 @@ int ensure_staging(Ctx* c, size_t bytes) {
   return LBM_OK;
 }
 
+void free_arrays(Ctx* c) {
+  void** ptrs[] = {reinterpret_cast<void**>(&c->fbuf[0]), reinterpret_cast<void**>(&c->fbuf[1]), &c->pop,
+                   reinterpret_cast<void**>(&c->mask),    reinterpret_cast<void**>(&c->flags),
+                   reinterpret_cast<void**>(&c->links),   reinterpret_cast<void**>(&c->rho),
+                   reinterpret_cast<void**>(&c->u),       reinterpret_cast<void**>(&c->status),
+                   reinterpret_cast<void**>(&c->partials), reinterpret_cast<void**>(&c->sums), &c->staging};
+  for (void** p : ptrs) {
+    if (*p) cudaFree(*p);
+    *p = nullptr;
+  }
+  c->dev_bytes = 0;
+}
+
 void free_all(Ctx* c) {
   for (auto& g : c->graph)
     if (g) cudaGraphExecDestroy(g);
-  void* ptrs[] = {c->fbuf[0], c->fbuf[1], c->pop,      c->mask,     c->flags, c->links,
-                  c->rho,     c->u,       c->status,   c->partials, c->sums,  c->staging};
-  for (void* p : ptrs)
-    if (p) cudaFree(p);
+  free_arrays(c);
   if (c->own_stream) cudaStreamDestroy(c->own_stream);
 }
 
@@ -262,9 +272,8 @@ int lbm_create(const lbm_desc* desc, lbm_ctx** out) {
     p.u_round = desc->ref_u_round;
   } else {
     // periodic rows are padded for the row tiles where those may run (lbm_set_params
-    // can turn Smagorinsky on and off), and else, or where the padding does not fit,
-    // lie one behind the other
-    const size_t eb = lbm::elem_bytes(desc->precision);
+    // can turn Smagorinsky on and off), and else, or where the lattice does not fit
+    // with them padded (below), lie one behind the other
     bool rows = lbm::setup_physics(*c, *desc, true);
     if (rows) {
       lbm::PhysParams plain = c->pp, smag = c->pp;
@@ -272,24 +281,34 @@ int lbm_create(const lbm_desc* desc, lbm_ctx** out) {
       smag.smag_cs = 0.1f;
       rows = lbm::phys_rows_pay(plain, *desc) || lbm::phys_rows_pay(smag, *desc);
     }
-    for (;; rows = false) {
-      if (!rows && !lbm::setup_physics(*c, *desc, false))
-        return bail(fail(c, LBM_ERR_UNSUPPORTED, "padded grid exceeds 2^32 nodes per slot array"));
-      rc = dev_alloc(c, reinterpret_cast<char**>(&c->pop), 19 * c->pp.g.slot_stride * eb, "cudaMalloc(populations)");
-      if (!rc) break;
-      if (!rows || !desc->periodic[0] || rc != LBM_ERR_OUT_OF_MEMORY) return bail(rc);
-    }
+    if (!rows && !lbm::setup_physics(*c, *desc, false))
+      return bail(fail(c, LBM_ERR_UNSUPPORTED, "padded grid exceeds 2^32 nodes per slot array"));
   }
   c->nblk_cons = lbm::cons_blocks(n);
-  if ((rc = dev_alloc(c, &c->mask, n, "cudaMalloc(mask)")) ||
-      (rc = dev_alloc(c, &c->flags, n, "cudaMalloc(flags)")) ||
-      (rc = dev_alloc(c, &c->links, n, "cudaMalloc(links)")) ||
-      (rc = dev_alloc(c, &c->rho, n, "cudaMalloc(rho)")) ||
-      (rc = dev_alloc(c, &c->u, 3 * n, "cudaMalloc(u)")) ||
-      (rc = dev_alloc(c, &c->status, 4, "cudaMalloc(status)")) ||
-      (rc = dev_alloc(c, &c->partials, 4 * (size_t)c->nblk_cons, "cudaMalloc(partials)")) ||
-      (rc = dev_alloc(c, &c->sums, 4 + (c->pop ? lbm::CLO_FRAG_WORDS / 2 : 0), "cudaMalloc(sums)")))
-    return bail(rc);
+  const bool physics = desc->mode == LBM_MODE_PHYSICS;
+  auto arrays = [&]() -> int {
+    int r = LBM_OK;
+    if ((physics && (r = dev_alloc(c, reinterpret_cast<char**>(&c->pop),
+                                   19 * c->pp.g.slot_stride * lbm::elem_bytes(desc->precision),
+                                   "cudaMalloc(populations)"))) ||
+        (r = dev_alloc(c, &c->mask, n, "cudaMalloc(mask)")) ||
+        (r = dev_alloc(c, &c->flags, n, "cudaMalloc(flags)")) ||
+        (r = dev_alloc(c, &c->links, n, "cudaMalloc(links)")) ||
+        (r = dev_alloc(c, &c->rho, n, "cudaMalloc(rho)")) ||
+        (r = dev_alloc(c, &c->u, 3 * n, "cudaMalloc(u)")) ||
+        (r = dev_alloc(c, &c->status, 4, "cudaMalloc(status)")) ||
+        (r = dev_alloc(c, &c->partials, 4 * (size_t)c->nblk_cons, "cudaMalloc(partials)")) ||
+        (r = dev_alloc(c, &c->sums, 4 + (physics ? lbm::CLO_FRAG_WORDS / 2 : 0), "cudaMalloc(sums)")))
+      return r;
+    return LBM_OK;
+  };
+  rc = arrays();
+  if (rc == LBM_ERR_OUT_OF_MEMORY && physics && c->pp.g.per[0] && c->pp.g.px > desc->nx) {
+    free_arrays(c);
+    lbm::setup_physics(*c, *desc, false);
+    rc = arrays();
+  }
+  if (rc) return bail(rc);
   if (c->pop) c->clo_frag = c->sums + 4;  // behind the sums: lbm_set_closure allocates nothing
 
   cudaStream_t s = c->stream;
