@@ -272,15 +272,16 @@ int lbm_create(const lbm_desc* desc, lbm_ctx** out) {
     p.u_round = desc->ref_u_round;
   } else {
     // periodic rows are padded for the row tiles where those may run (lbm_set_params
-    // can turn Smagorinsky on and off), and else, or where the lattice does not fit
-    // with them padded (below), lie one behind the other
-    bool rows = lbm::setup_physics(*c, *desc, true);
-    if (rows) {
-      lbm::PhysParams plain = c->pp, smag = c->pp;
-      plain.smag_cs = 0.f;
-      smag.smag_cs = 0.1f;
-      rows = lbm::phys_rows_pay(plain, *desc) || lbm::phys_rows_pay(smag, *desc);
-    }
+    // can turn Smagorinsky and a body force on and off), and else, or where the
+    // lattice does not fit with them padded (below), lie one behind the other
+    bool rows = false;
+    if (lbm::setup_physics(*c, *desc, true))
+      for (int k = 0; k < 4; ++k) {
+        lbm::PhysParams p = c->pp;
+        p.smag_cs = k & 1 ? 0.1f : 0.f;
+        for (float& a : p.accel) a = k & 2 ? 1e-6f : 0.f;
+        rows = rows || lbm::phys_rows_pay(p, *desc);
+      }
     if (!rows && !lbm::setup_physics(*c, *desc, false))
       return bail(fail(c, LBM_ERR_UNSUPPORTED, "padded grid exceeds 2^32 nodes per slot array"));
   }

@@ -128,3 +128,21 @@ def test_lanes_run_and_equal_single_domains(gpu, name):
     b.set_schedule(persistent=1)
     assert b.lanes(1000) == 0
     b.close()
+
+
+@pytest.mark.parametrize("prec,shape,trt,cs,forced,plain", [
+    (2, (77, 63, 81), True, 0.0, True, False), (1, (257, 80, 101), False, 0.1, True, False),
+    (0, (149, 57, 46), True, 0.1, False, True), (0, (201, 48, 75), True, 0.1, True, False)])
+def test_odd_rows_with_a_force_have_their_own_lines(gpu, prec, shape, trt, cs, forced, plain):
+    """The two kernels round the half force differently, so the lines of odd
+    forced rows are apart from the others': `forced` with a body force along x,
+    `plain` without."""
+    force, none = (1e-6, 0.0, 0.0), (0.0, 0.0, 0.0)
+    for accel, want, other, want_other in ((force, forced, none, plain), (none, plain, force, forced)):
+        lat = gpu.Lattice(nx=shape[0], ny=shape[1], nz=shape[2], mode=gpu.MODE_PHYSICS, precision=prec,
+                          collision=gpu.COLL_TRT if trt else gpu.COLL_BGK, periodic=(1, 0, 1), tau=0.57,
+                          smagorinsky_cs=cs, body_accel=accel)
+        assert lat.streams_rows() == want
+        lat.set_params(body_accel=other)
+        assert lat.streams_rows() == want_other
+        lat.close()
