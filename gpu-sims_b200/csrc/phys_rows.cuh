@@ -805,13 +805,14 @@ inline uint32_t rows_chip_blocks(const PhysGeom& G, int precision, bool smag) {
 //  * rows below 66 nodes waste padding and tiles: 64^3 fp16 22.8 against 30.2 GLUPS.
 // Open x faces cost the row kernels a launch of their own: 128^3 fp16 with
 // Smagorinsky 0.82, without the faces 1.03.
-// Odd rows with a body force have lines of their own (`fill` and the number of
-// tiles), which time alone does not draw: the one-node kernel rounds j / rho and the
-// half force apart, the packed collision here in one multiply-add, and 2-byte
-// stores carry that into results 2e-3 apart after 50 steps, so a line moved is a
-// result changed.  On both sides of them a time is lost: bf16 77 x 63 x 81 TRT 0.87,
-// fp32 with Smagorinsky 437 x 97 x 46 0.90 and 201 x 48 x 75 1.13, fp16 with
-// Smagorinsky 257 x 80 x 101 1.24 of the row kernels' time.
+// A body force where the one-node kernel would run (odd rows, even ones that are no
+// pairs', open faces) has lines of its own (`fill` and the number of tiles), which
+// time alone does not draw: that kernel rounds j / rho and the half force apart, the
+// packed collision here in one multiply-add, and 2-byte stores carry that into
+// results 2e-3 apart after 50 steps, so a line moved is a result changed.  On both
+// sides of them a time is lost: bf16 77 x 63 x 81 TRT 0.87, fp32 with Smagorinsky 437
+// x 97 x 46 0.90 and 201 x 48 x 75 1.13, fp16 with Smagorinsky 257 x 80 x 101 1.24 of
+// the row kernels' time.
 // Inside the other lines 1 in 50 of the timings is slower by more than 4 per cent,
 // the worst by 10 (81 x 97 x 120, periodic, TRT, Smagorinsky, fp32, single steps).
 inline bool row_tiles_pay(const PhysParams& p, const lbm_desc& d) {
@@ -824,7 +825,8 @@ inline bool row_tiles_pay(const PhysParams& p, const lbm_desc& d) {
   const int fill = 100 * rt.R * G.nx / 512;  // per cent of a tile
   if (f32 ? fill < 74 : !odd && fill < 76) return false;
   const uint32_t nt = rt.ntiles, blocks = rows_chip_blocks(G, d.precision, smag);
-  if (odd && (p.accel[0] != 0.f || p.accel[1] != 0.f || p.accel[2] != 0.f)) return nt >= (f32 ? 1000u : 700u);
+  const bool force = p.accel[0] != 0.f || p.accel[1] != 0.f || p.accel[2] != 0.f;
+  if (force && (!step_pairs(G.nx) || p.any_open)) return nt >= (whole ? (f32 ? 12000u : 4000u) : (f32 ? 1000u : 700u));
   // per mille
   const int used = (int)(1000 * (uint64_t)G.n / (512ull * blocks * ((nt + blocks - 1) / blocks)));
   if (rt.tiles_y < (whole ? 12 : smag || rt.R < 5 ? 5 : 3)) return false;

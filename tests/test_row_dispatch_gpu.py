@@ -132,11 +132,12 @@ def test_lanes_run_and_equal_single_domains(gpu, name):
 
 @pytest.mark.parametrize("prec,shape,trt,cs,forced,plain", [
     (2, (77, 63, 81), True, 0.0, True, False), (1, (257, 80, 101), False, 0.1, True, False),
-    (0, (149, 57, 46), True, 0.1, False, True), (0, (201, 48, 75), True, 0.1, True, False)])
-def test_odd_rows_with_a_force_have_their_own_lines(gpu, prec, shape, trt, cs, forced, plain):
-    """The two kernels round the half force differently, so the lines of odd
-    forced rows are apart from the others': `forced` with a body force along x,
-    `plain` without."""
+    (0, (149, 57, 46), True, 0.1, False, True), (0, (201, 48, 75), True, 0.1, True, False),
+    (1, (88, 10, 400), False, 0.0, True, False), (0, (256, 10, 3000), False, 0.0, False, False)])
+def test_a_force_on_one_node_rows_has_its_own_lines(gpu, prec, shape, trt, cs, forced, plain):
+    """The one-node kernel rounds the half force differently, so the lines of
+    forced rows that it would take (odd, ragged) are apart from the others', and
+    those of the pair kernel are not: `forced` with a body force, `plain` without."""
     force, none = (1e-6, 0.0, 0.0), (0.0, 0.0, 0.0)
     for accel, want, other, want_other in ((force, forced, none, plain), (none, plain, force, forced)):
         lat = gpu.Lattice(nx=shape[0], ny=shape[1], nz=shape[2], mode=gpu.MODE_PHYSICS, precision=prec,
